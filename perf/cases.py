@@ -22,6 +22,7 @@ from starlab_b200.server import ResidentServer, Server
 from starlab_b200.story import StoryReader, format_story
 
 T_BLOCK = 1.0 / 128  # block time of the single calls; the j-state is at time 0
+LIST_MAX = 512       # neighbours read back per particle (a few tens are found)
 T_LAST = 1.0 / 256   # time of the previous block's corrected particles
 
 
@@ -164,23 +165,33 @@ def _block(case, seed):
     return m, x, v, a, j, last, members, xl, vl
 
 
-def _sizes(case, seed):
-    rng = np.random.default_rng(seed)
+def _spread(count, salt):
+    """`count` values evenly spread over [0, 1), jittered, in no order."""
+    rng = np.random.default_rng(salt)
+    return (rng.permutation(count) + rng.uniform(0.0, 1.0, count)) / count
+
+
+def _sizes(case):
+    """The clusters' sizes, log-uniform: the case's own, the same for every seed."""
     lo, hi = math.log(case["n_lo"]), math.log(case["n_hi"])
-    # evenly spread over the logarithm, jittered: the total hardly depends on the seed
-    u = (np.arange(case["clusters"]) + rng.uniform(0.0, 1.0, case["clusters"])) / case["clusters"]
-    return np.exp(lo + u * (hi - lo)).astype(int)
+    return np.exp(lo + _spread(case["clusters"], case["n_hi"]) * (hi - lo)).astype(int)
+
+
+def _call_sizes(case):
+    """(cluster, its n, ni) of each call of a burst, ni from p(ni) ~ 1/ni."""
+    ns, u = _sizes(case), _spread(case["calls"], case["n_hi"] + 1)
+    out = []
+    for q in range(case["calls"]):
+        n = int(ns[q % len(ns)])
+        out.append((q % len(ns), n, min(n, max(1, int(math.exp(u[q] * math.log(n)))))))
+    return out
 
 
 def _served(case, seed):
-    clusters = [_cluster(int(n), 1000 * seed + k) for k, n in enumerate(_sizes(case, seed))]
+    clusters = [_cluster(int(n), 1000 * seed + k) for k, n in enumerate(_sizes(case))]
     rng = np.random.default_rng(seed + 3)
     calls = []
-    u = (rng.permutation(case["calls"]) + rng.uniform(0.0, 1.0, case["calls"])) / case["calls"]
-    for q in range(case["calls"]):
-        c = (q * 7 + 3) % len(clusters)
-        n = len(clusters[c][0])
-        ni = min(n, max(1, int(math.exp(u[q] * math.log(n)))))
+    for q, (c, n, ni) in enumerate(_call_sizes(case)):
         i0 = int(rng.integers(0, n - ni + 1))
         ti = 1e-5 * (q + 1)
         _, x, v, a, j = clusters[c]
@@ -214,7 +225,7 @@ def prepare(case, seed):
         return {"case": case, "h3": H3Engine(), "n": case["n"], "m": m, "x": x, "v": v,
                 "a2": 0.5 * a, "j6": j / 6.0}
     if kind == "ensemble":
-        ns = _sizes(case, seed)
+        ns = _sizes(case)
         cl = [ics.plummer(int(n), 1000 * seed + k) for k, n in enumerate(ns)]
         ens = Ensemble([c[0] for c in cl], [c[1] for c in cl], [c[2] for c in cl], (4.0 / ns) ** 2, eta=0.02,
                        precision=case["precision"])
@@ -253,9 +264,11 @@ def run(state):
         if not lists:
             return {"acc": acc, "jerk": jerk, "pot": pot, "nn": nn}
         eng.read_neighbour_list()
-        got = [eng.get_neighbour_list(p)[1] for p in range(case["ni"])]
-        return {"acc": acc, "jerk": jerk, "pot": pot, "nn": nn,
-                "count": np.array([len(g) for g in got], np.int32), "lists": np.concatenate(got)}
+        count, rows = np.empty(case["ni"], np.int32), np.full((case["ni"], LIST_MAX), -1, np.int32)
+        for p in range(case["ni"]):
+            got = eng.get_neighbour_list(p, LIST_MAX)[1]
+            count[p], rows[p, :len(got)] = len(got), got
+        return {"acc": acc, "jerk": jerk, "pot": pot, "nn": nn, "count": count, "lists": rows}
     if kind in ("sweep", "energies"):
         eng = state["h"].eng
         eng.set_j_particles(0.0, state["m"], state["j6"], state["a2"], state["v"], state["x"])
@@ -320,14 +333,12 @@ def work(case):
     if kind == "ensemble":
         # every particle's state in and out, and at least one force on each
         # at t = 0 and at each of the largest steps (1/16 at most) after it
-        ns = _sizes(case, 0)
+        ns = _sizes(case)
         return {"bytes": int(ns.sum()) * (56 + 14 * 8), "flops": PAIR_FLOPS * 2.0 * float((ns.astype(float) ** 2).sum())}
     if kind == "served":
-        ns = _sizes(case, 0)
-        n = [int(ns[(q * 7 + 3) % len(ns)]) for q in range(case["calls"])]
-        ni = [(k - 1) / math.log(k) for k in n]  # the mean of p(ni) ~ 1/ni
-        return {"bytes": sum(J_BYTES * k + (I_BYTES + OUT_BYTES) * i for k, i in zip(n, ni)),
-                "flops": PAIR_FLOPS * sum(k * i for k, i in zip(n, ni))}
+        calls = _call_sizes(case)
+        return {"bytes": sum(J_BYTES * n + (I_BYTES + OUT_BYTES) * ni for _, n, ni in calls),
+                "flops": PAIR_FLOPS * sum(n * ni for _, n, ni in calls)}
     return {"bytes": (275 + 56) * case["n"], "flops": 0}
 
 
