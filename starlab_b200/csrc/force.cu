@@ -158,8 +158,12 @@ static KernelFn pick3(bool nb, bool ident) {
 template <int K>
 static KernelFn pick2(int il, int r, bool nb, bool ident) {
     if (il == 32) {
-        if (K == kKernMixedDS && r == 4) return pick3<K, 32, 4>(nb, ident);
-        if (K != kKernMixedP && r == 2) return pick3<K, 32, 2>(nb, ident);
+        if constexpr (K == kKernMixedDS) {
+            if (r == 4) return pick3<K, 32, 4>(nb, ident);
+        }
+        if constexpr (K != kKernMixedP) {
+            if (r == 2) return pick3<K, 32, 2>(nb, ident);
+        }
         return pick3<K, 32, 1>(nb, ident);
     }
     if (il == 8) return pick3<K, 8, 1>(nb, ident);

@@ -18,6 +18,19 @@ constexpr uint64_t kWaitLimitNs = 1000000000ull;  // 1 s per tile wait
 constexpr int kFlush = G6B200_FOLD_TERMS;         // FP32 terms per FP64 fold
 constexpr int kMaxWarps = 8;
 
+// Variant bits of the mixed kernels: 2 = inner j-loop of the scalar layout
+// unrolled by 4 (else 2): 1.3% faster.  (The paired layout's loop is
+// unrolled by 16 with the indicators on, by 4 otherwise.)
+constexpr int kVarUnroll4 = 2;
+// 4 = GRAPE-4 pipeline (FP64 kernel only; see the file header).
+constexpr int kVarG4 = 4;
+// 8 = potential only (paired mixed and FP64 layouts): the energy sweeps.
+constexpr int kVarPot = 8;
+// 16 = paired mixed layout: also track the refinement's error indicators
+// (the largest single acc and jerk terms: one FP32x2 multiply and two
+// three-input integer maxima per pair of j).
+constexpr int kVarStats = 16;
+
 // T j per shared-memory tile, held as U records of JPU j each.
 template <int K> struct Traits;
 template <> struct Traits<kKernMixedDS> {
@@ -32,6 +45,8 @@ template <> struct Traits<kKernF64> {
     using JRec = JRecF64;
     static constexpr int T = 128, JPU = 1, U = T;
 };
+
+constexpr unsigned kHiInf = 0x7ff00000u;  // upper word of the FP64 +inf
 
 // Per-i register state.
 
@@ -49,8 +64,11 @@ struct StateMixed : StateMixedBase {
 
 struct StateF64 {
     double x, y, z, vx, vy, vz, h2;
-    double eps2;  // per-i softening (GRAPE-4 variant only)
-    double Ax, Ay, Az, Jx, Jy, Jz, Pt;
+    double eps2;  // softening: the call's, or (GRAPE-4 variant) this i's
+    double Ax, Ay, Az, Jx, Jy, Jz, Pt;  // acc, jerk x 3 sqrt(3), pot x sqrt(3): see inv_dist_s3
+    unsigned nhi;  // smallest upper word of r^2 so far
+    int nk;        // first j of the run that first reached it (-1: none)
+    bool ntie;     // another run reached the same upper word
     double nr2;
     int nj, idx, i;
 };
@@ -83,7 +101,7 @@ __device__ __forceinline__ void load_i(StateMixed &s, const IRec &q, const Force
     init_mixed(s, q);
 }
 
-__device__ __forceinline__ void load_i(StateF64 &s, const IRec &q, const ForceParams &, bool &) {
+__device__ __forceinline__ void load_i(StateF64 &s, const IRec &q, const ForceParams &p, bool &) {
     s.x = q.x[0];
     s.y = q.x[1];
     s.z = q.x[2];
@@ -92,7 +110,11 @@ __device__ __forceinline__ void load_i(StateF64 &s, const IRec &q, const ForcePa
     s.vz = q.v[2];
     s.h2 = q.h2;
     s.idx = q.index;
+    s.eps2 = p.eps2;
     s.Ax = s.Ay = s.Az = s.Jx = s.Jy = s.Jz = s.Pt = 0.0;
+    s.nhi = kHiInf;
+    s.nk = -1;
+    s.ntie = false;
     s.nr2 = DBL_MAX;
     s.nj = -1;
 }
@@ -158,88 +180,153 @@ __device__ __forceinline__ void interact_mixed(S &s, const JMixed &J, int jg, fl
     }
 }
 
-template <bool CHK, bool NB, bool IDENT, bool G4 = false, bool PO = false>
-__device__ __forceinline__ void interact(StateF64 &s, const double4 &pos, const double4 &vel,
-                                         int jg, double eps2, const ForceParams &p) {
-    if constexpr (PO) {
-        // Potential only: the pot term of the full form below.
-        const double dx = pos.x - s.x;
-        const double dy = pos.y - s.y;
-        const double dz = pos.z - s.z;
-        double r2 = dx * dx + dy * dy + dz * dz + eps2;
-        double mj = pos.w;
-        if (CHK) {
-            const bool self = IDENT ? (jg == s.idx) : ((int)vel.w == s.idx);
-            r2 = self ? 1.0 : r2;
-            mj = self ? 0.0 : mj;
-        }
-        s.Pt -= mj * rsqrt(r2);
-        return;
+// ---- FP64 layout.
+//
+// What bounds this loop is the register ports: a scheduler reads one 64-bit
+// register operand per cycle for its warp, so an FP64 instruction with three
+// different register operands takes 3 cycles, one with two takes the FP64
+// pipe's 2 (measured: 3.04 and 2.04; an operand shared with the previous
+// instruction, or a literal one, is free).  The loop below is written
+// against that count -- about 70 cycles per j and warp:
+//   * the inverse distance is the PTX approximation and one third-order step
+//     in line (11 cycles; rsqrt() measured 26, with a branch for the special
+//     values that keeps the pair terms of neighbouring j apart);
+//   * it is scaled by sqrt(3), so that 3 (dr.dv) / r^2 needs no product of
+//     its own;
+//   * the nearest neighbour is kept as the upper word of r^2 (one integer
+//     minimum per j instead of an FP64 compare and three selects).
+// 16384 x 262144: 10.56 -> 9.21 ms; potential only, 65536 x 65536: 5.39 ->
+// 3.69 ms.
+constexpr double kSqrt3 = 1.7320508075688772935;
+constexpr double kThird = 1.0 / 3.0;
+
+// sqrt(3) / r from r^2 / 3 (finite, normal, positive): the approximation's
+// relative error e/2, e = 1 - x y^2 below 2^-18, goes to 5/16 e^3 by
+// Householder's third-order step for x^(-1/2) (A. S. Householder, "The
+// Numerical Treatment of a Single Nonlinear Equation", 1970), y (1 + e/2 +
+// 3/8 e^2): below FP64's rounding.
+__device__ __forceinline__ double inv_dist_s3(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-(x * y), y, 1.0);
+    return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+
+__device__ __forceinline__ double r2_f64(double dx, double dy, double dz) {
+    return __fma_rn(dz, dz, __fma_rn(dy, dy, dx * dx));
+}
+
+template <bool IDENT>
+__device__ __forceinline__ bool is_self(const StateF64 &s, const double4 &vel, int jg) {
+    return IDENT ? jg == s.idx : vel.w == (double)s.idx;
+}
+
+// One pair term for any r^2 (zero, subnormal and infinite ones too).
+template <bool CHK, bool IDENT, bool G4, bool PO>
+__device__ __forceinline__ void interact_any(StateF64 &s, const double4 &pos, const double4 &vel, int jg) {
+    const double dx = pos.x - s.x, dy = pos.y - s.y, dz = pos.z - s.z;
+    double r2 = G4 ? g4_r2(dx, dy, dz, s.eps2) : r2_f64(dx, dy, dz) + s.eps2;
+    double mj = pos.w;
+    if (G4 ? !(r2 > 0.0) : (CHK && is_self<IDENT>(s, vel, jg))) {
+        r2 = 1.0;
+        mj = 0.0;
     }
-    const double dx = pos.x - s.x;
-    const double dy = pos.y - s.y;
-    const double dz = pos.z - s.z;
-    const double dvx = vel.x - s.vx;
-    const double dvy = vel.y - s.vy;
-    const double dvz = vel.z - s.vz;
-    const double rv = dx * dvx + dy * dvy + dz * dvz;
-    if (G4) {
-        // The same rounding sequence as g4_r2() in the neighbour-list pass.
-        double r2 = g4_r2(dx, dy, dz, s.eps2);
-        if (NB && r2 < s.h2) nb_push(p, s.i, jg);
-        const bool zero = !(r2 > 0.0);
-        const double mj = zero ? 0.0 : pos.w;
-        const double r2nn = zero ? DBL_MAX : r2;
-        r2 = zero ? 1.0 : r2;
-        const double rinv = rsqrt(r2);
+    const double rinv = rsqrt(r2);
+    const double mr = mj * rinv;
+    s.Pt -= kSqrt3 * mr;
+    if constexpr (!PO) {
+        const double dvx = vel.x - s.vx, dvy = vel.y - s.vy, dvz = vel.z - s.vz;
+        const double rv = dx * dvx + dy * dvy + dz * dvz;
         const double r2inv = rinv * rinv;
-        const double mr = mj * rinv;
-        const double mr3 = mr * r2inv;
+        const double mr3 = (3.0 * kSqrt3) * (mr * r2inv);
         const double a3 = -3.0 * rv * r2inv;
-        s.Pt -= mr;
         s.Ax += mr3 * dx;
         s.Ay += mr3 * dy;
         s.Az += mr3 * dz;
         s.Jx += mr3 * (dvx + a3 * dx);
         s.Jy += mr3 * (dvy + a3 * dy);
         s.Jz += mr3 * (dvz + a3 * dz);
-        if (r2nn < s.nr2) {
-            s.nr2 = r2nn;
-            s.nj = jg;
-        }
-        return;
     }
-    const double r2n = dx * dx + dy * dy + dz * dz;
-    double r2 = r2n + eps2;
-    double mj = pos.w;
-    double r2nn = r2n;
+}
+
+// One pair term, r^2 / 3 taken as finite, normal and positive (the caller
+// sums again with interact_any when it was not: the sums then are not
+// finite).  Returns the upper word of the unsoftened r^2 (all ones for the
+// particle itself).
+template <bool CHK, bool NB, bool IDENT, bool G4, bool PO>
+__device__ __forceinline__ unsigned interact(StateF64 &s, const JRecF64 &J, int jg, const ForceParams &p) {
+    const double dx = J.pos.x - s.x, dy = J.pos.y - s.y, dz = J.pos.z - s.z;
+    double r2 = G4 ? g4_r2(dx, dy, dz, s.eps2) : r2_f64(dx, dy, dz);
+    double m = J.pos.w;
+    unsigned hi = (unsigned)__double2hiint(r2);
     bool self = false;
-    if (CHK) {
-        self = IDENT ? (jg == s.idx) : ((int)vel.w == s.idx);
-        r2 = self ? 1.0 : r2;
-        mj = self ? 0.0 : mj;
-        r2nn = self ? DBL_MAX : r2nn;
-    }
-    const double rinv = rsqrt(r2);
-    const double r2inv = rinv * rinv;
-    const double mr = mj * rinv;
-    const double mr3 = mr * r2inv;
-    const double a3 = -3.0 * rv * r2inv;
-    s.Pt -= mr;
-    s.Ax += mr3 * dx;
-    s.Ay += mr3 * dy;
-    s.Az += mr3 * dz;
-    s.Jx += mr3 * (dvx + a3 * dx);
-    s.Jy += mr3 * (dvy + a3 * dy);
-    s.Jz += mr3 * (dvz + a3 * dz);
-    if (r2nn < s.nr2) {
-        s.nr2 = r2nn;
-        s.nj = jg;
-    }
+    if (CHK && !G4) self = is_self<IDENT>(s, J.vel, jg);
     if (NB) {
-        bool hit = CHK && self ? (p.include_self && s.h2 > 0.0) : (r2n < s.h2);
+        const bool hit = CHK && self ? (p.include_self && s.h2 > 0.0) : (r2 < s.h2);
         if (hit) nb_push(p, s.i, jg);
     }
+    if (CHK || G4) {
+        // left out: m = 0 at r = 1 (GRAPE-4: r^2 = 0)
+        const bool out = G4 ? (hi | (unsigned)__double2loint(r2)) == 0u : self;
+        m = out ? 0.0 : m;
+        r2 = out ? 1.0 : r2;
+        hi = out ? 0xffffffffu : hi;
+    }
+    const double y = inv_dist_s3(G4 ? r2 * kThird : __fma_rn(r2, kThird, s.eps2 * kThird));
+    if constexpr (PO) {
+        s.Pt = __fma_rn(-m, y, s.Pt);
+        return hi;
+    }
+    const double dvx = J.vel.x - s.vx, dvy = J.vel.y - s.vy, dvz = J.vel.z - s.vz;
+    const double rv = __fma_rn(dz, dvz, __fma_rn(dy, dvy, dx * dvx));
+    const double q3 = y * y;  // 3 / r^2
+    const double mr = m * y;
+    const double mr3 = mr * q3;
+    const double a3 = rv * q3;
+    s.Pt -= mr;
+    s.Ax = __fma_rn(mr3, dx, s.Ax);
+    s.Ay = __fma_rn(mr3, dy, s.Ay);
+    s.Az = __fma_rn(mr3, dz, s.Az);
+    s.Jx = __fma_rn(mr3, __fma_rn(-a3, dx, dvx), s.Jx);
+    s.Jy = __fma_rn(mr3, __fma_rn(-a3, dy, dvy), s.Jy);
+    s.Jz = __fma_rn(mr3, __fma_rn(-a3, dz, dvz), s.Jz);
+    return hi;
+}
+
+// Nearest neighbour of the FP64 kernels: the j of [j0, j0 + n JL) in steps
+// of JL (addresses) with the smallest unsoftened r^2, the first on a tie.
+// Of a run, up to eight records are loaded before the first is used.
+template <int JL, bool IDENT>
+__device__ __forceinline__ void nn_scan_one(StateF64 &s, const double4 &pos, double w, int jg) {
+    const double r2 = r2_f64(pos.x - s.x, pos.y - s.y, pos.z - s.z);
+    const bool self = IDENT ? jg == s.idx : w == (double)s.idx;
+    if (!self && r2 < s.nr2) {
+        s.nr2 = r2;
+        s.nj = jg;
+    }
+}
+
+template <int JL, int RUN, bool IDENT>
+__device__ __forceinline__ void nn_scan_run(StateF64 &s, const JRecF64 *src, int j0) {
+    constexpr int B = RUN < 8 ? RUN : 8;
+#pragma unroll 1
+    for (int b = 0; b < RUN; b += B) {
+        double4 pos[B];
+        double w[B];
+#pragma unroll
+        for (int u = 0; u < B; ++u) {
+            pos[u] = src[j0 + (b + u) * JL].pos;
+            w[u] = IDENT ? 0.0 : src[j0 + (b + u) * JL].vel.w;
+        }
+#pragma unroll
+        for (int u = 0; u < B; ++u) nn_scan_one<JL, IDENT>(s, pos[u], w[u], j0 + (b + u) * JL);
+    }
+}
+
+template <int JL, bool IDENT>
+__device__ __forceinline__ void nn_scan(StateF64 &s, const JRecF64 *jrec, int j0, int n) {
+#pragma unroll 1
+    for (int u = 0; u < n; ++u) nn_scan_one<JL, IDENT>(s, jrec[j0 + u * JL].pos, jrec[j0 + u * JL].vel.w, j0 + u * JL);
 }
 
 // ---- paired layout: one FP32x2 instruction evaluates i against two j.
@@ -423,18 +510,17 @@ __device__ __forceinline__ void fold(StateMixedBase &s) {
     s.ax = s.ay = s.az = s.jx = s.jy = s.jz = s.pt = 0.f;
 }
 
-// Variant bits of the mixed kernels: 2 = inner j-loop of the scalar layout
-// unrolled by 4 (else 2): 1.3% faster.  (The paired layout's loop is
-// unrolled by 16 with the indicators on, by 4 otherwise.)
-constexpr int kVarUnroll4 = 2;
-// 4 = GRAPE-4 pipeline (FP64 kernel only; see the file header).
-constexpr int kVarG4 = 4;
-// 8 = potential only (paired mixed and FP64 layouts): the energy sweeps.
-constexpr int kVarPot = 8;
-// 16 = paired mixed layout: also track the refinement's error indicators
-// (the largest single acc and jerk terms: one FP32x2 multiply and two
-// three-input integer maxima per pair of j).
-constexpr int kVarStats = 16;
+// The nearest neighbour in two steps (FP64 kernels): the pair loop keeps a
+// minimum alone, and after every run of NnRun records it is compared with
+// its value before the run, so the run that first reached the minimum is
+// known.  At the end of the task that run's records are looked through again
+// (nn_scan_run): the same j as a compare and select in every pair term.  A
+// run divides a thread's share of a tile (a multiple of 16 records at 32
+// i-lanes, 4 at 8 i-lanes, any number at 1).
+template <int K, int JL, int R, int V> struct NnRun {
+    static constexpr int value =
+        JL == 1 ? (K == kKernF64 && (R == 2 || (V & (kVarG4 | kVarPot)) != 0) ? 16 : 8) : (JL == 4 ? 4 : 1);
+};
 
 // Consume one shared-memory tile: this thread's j are kbase + m*JL.
 template <int K, int R, int JL, bool CHK, bool NB, bool IDENT, int V>
@@ -492,15 +578,33 @@ __device__ __forceinline__ void consume_tile(typename StateOf<K>::type (&st)[R],
             for (int r = 0; r < R; ++r) fold_any<PO>(st[r]);
         }
     } else if constexpr (K == kKernF64) {
-        const double eps2 = p.eps2;
-#pragma unroll 2
-        for (int m = 0; m < per; ++m) {
-            const int k = kbase + m * JL;
-            const double4 pos = S[k].pos;
-            const double4 vel = S[k].vel;
+        constexpr bool G4 = (V & kVarG4) != 0, PO = (V & kVarPot) != 0;
+        constexpr int RUN = NnRun<K, JL, R, V>::value;
+        for (int m0 = 0; m0 < per; m0 += RUN) {
+            unsigned lo[R];
 #pragma unroll
-            for (int r = 0; r < R; ++r)
-                interact<CHK, NB, IDENT, (V & kVarG4) != 0, (V & kVarPot) != 0>(st[r], pos, vel, tb + k, eps2, p);
+            for (int r = 0; r < R; ++r) lo[r] = 0xffffffffu;
+#pragma unroll
+            for (int u = 0; u < RUN; ++u) {
+                const int k = kbase + (m0 + u) * JL;
+                const JRecF64 J = S[k];
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                    lo[r] = min(lo[r], interact<CHK, NB, IDENT, G4, PO>(st[r], J, tb + k, p));
+            }
+            // the GRAPE-4 pipeline returns no neighbour index
+            if constexpr (!G4 && !PO) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    if (lo[r] < st[r].nhi) {
+                        st[r].nhi = lo[r];
+                        st[r].nk = tb + kbase + m0 * JL;
+                        st[r].ntie = false;
+                    } else if (lo[r] == st[r].nhi) {
+                        st[r].ntie = true;
+                    }
+                }
+            }
         }
     } else {
         const float eps2 = (float)p.eps2;
@@ -562,9 +666,10 @@ __device__ __forceinline__ void to_partial(const StateMixedP &s, Partial &q) {
     q.qj = __int_as_float(s.qj);          // max m / r^3
 }
 __device__ __forceinline__ void to_partial(const StateF64 &s, Partial &q) {
-    q.acc[0] = s.Ax; q.acc[1] = s.Ay; q.acc[2] = s.Az;
-    q.jerk[0] = s.Jx; q.jerk[1] = s.Jy; q.jerk[2] = s.Jz;
-    q.pot = s.Pt;
+    constexpr double c1 = 1.0 / kSqrt3, c3 = c1 / 3.0;
+    q.acc[0] = c3 * s.Ax; q.acc[1] = c3 * s.Ay; q.acc[2] = c3 * s.Az;
+    q.jerk[0] = c3 * s.Jx; q.jerk[1] = c3 * s.Jy; q.jerk[2] = c3 * s.Jz;
+    q.pot = c1 * s.Pt;
     q.nn_r2 = s.nr2;
     q.nn_j = s.nj;
     q.qa = q.qj = 0.f;
@@ -749,13 +854,46 @@ __device__ __forceinline__ bool process_task(const ForceParams &p, int itile_idx
     }
 
     // ---- epilogue: lanes -> warps -> (output | split partial)
+    // Records of the last two tiles are still in shared memory, the others
+    // are read where they came from.
+    constexpr int RUN = NnRun<K, JL, R, V>::value;
+    constexpr bool kRunNn = K == kKernF64 && (V & (kVarG4 | kVarPot)) == 0;
+    auto records_of = [&](int unit) -> const JRec * {
+        const int t2 = (unit * JPU - jb) / T;
+        return t2 >= ntiles - 2 ? tiles + ((g0 + t2) & 1) * U - (jb + t2 * T) / JPU : jrec;
+    };
     Partial q[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
+        if constexpr (K == kKernF64) {
+            const int first = jb + kbase;
+            // A sum that is not finite: some r^2 overflowed, vanished, or is
+            // negative or NaN.  Summed again with the pair term for any r^2.
+            if (!(fabs(st[r].Pt) <= DBL_MAX)) {
+                st[r].Ax = st[r].Ay = st[r].Az = st[r].Jx = st[r].Jy = st[r].Jz = st[r].Pt = 0.0;
+#pragma unroll 1
+                for (int t2 = 0; t2 < ntiles; ++t2)
+#pragma unroll 1
+                    for (int m = 0; m < per; ++m) {
+                        const int jg = first + t2 * T + m * JL;
+                        interact_any<true, IDENT, (V & kVarG4) != 0, (V & kVarPot) != 0>(st[r], jrec[jg].pos,
+                                                                                        jrec[jg].vel, jg);
+                    }
+            }
+            if constexpr (kRunNn) {
+                if (st[r].ntie) {
+#pragma unroll 1
+                    for (int t2 = 0; t2 < ntiles; ++t2) nn_scan<JL, IDENT>(st[r], jrec, first + t2 * T, per);
+                } else if (st[r].nk >= 0) {
+                    nn_scan_run<JL, RUN, IDENT>(st[r], records_of(st[r].nk), st[r].nk);
+                }
+            }
+        }
         to_partial(st[r], q[r]);
         if (JL > 1) warp_reduce<IL>(q[r]);
     }
     if (H > 1) {
+        if (kRunNn) __syncthreads();  // the tile area was read above
         if (jl == 0) {
 #pragma unroll
             for (int r = 0; r < R; ++r) red[h * itile + islot + r * IL] = q[r];
