@@ -340,6 +340,7 @@ struct StateMixedP {
     int qj;                             // and of max m/r^3 (signed max: the self term's -0.0 never wins)
     double Ax, Ay, Az, Jx, Jy, Jz, Pt;
     float nr2;
+    int nk;  // first pair record of the run of records that first reached nr2 (-1: none)
     int nj, idx, i;
 };
 template <> struct StateOf<kKernMixedP> { using type = StateMixedP; };
@@ -367,7 +368,25 @@ __device__ __forceinline__ void load_i(StateMixedP &s, const IRec &q, const Forc
     s.qj = 0;
     s.Ax = s.Ay = s.Az = s.Jx = s.Jy = s.Jz = s.Pt = 0.0;
     s.nr2 = FLT_MAX;
+    s.nk = -1;
     s.nj = -1;
+}
+
+// Unsoftened squared distances of i to the two j of a record (the pair
+// terms' own operations in their order), FLT_MAX for the particle itself.
+template <bool IDENT>
+__device__ __forceinline__ float2 pair_nn_r2(const StateMixedP &s, const JPairMixed &rec, int jg0) {
+    const float4 hxy = rec.hxy, hzm = rec.hzm, lxy = rec.lxy, lzi = rec.lzi;
+    const float2 dx = __fadd2_rn(__fadd2_rn(make_float2(hxy.x, hxy.y), s.nxh),
+                                 __fadd2_rn(make_float2(lxy.x, lxy.y), s.nxl));
+    const float2 dy = __fadd2_rn(__fadd2_rn(make_float2(hxy.z, hxy.w), s.nyh),
+                                 __fadd2_rn(make_float2(lxy.z, lxy.w), s.nyl));
+    const float2 dz = __fadd2_rn(__fadd2_rn(make_float2(hzm.x, hzm.y), s.nzh),
+                                 __fadd2_rn(make_float2(lzi.x, lzi.y), s.nzl));
+    float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+    if (IDENT ? (jg0 == s.idx) : (__float_as_int(lzi.z) == s.idx)) r2.x = FLT_MAX;
+    if (IDENT ? (jg0 + 1 == s.idx) : (__float_as_int(lzi.w) == s.idx)) r2.y = FLT_MAX;
+    return r2;
 }
 
 template <bool CHK, bool NB, bool IDENT, bool PO = false, bool STATS = false>
@@ -459,13 +478,17 @@ __device__ __forceinline__ void interact_pair(StateMixedP &s, const JPairMixed &
     s.jx = __ffma2_rn(mr3, __ffma2_rn(a3, dx, dvx), s.jx);
     s.jy = __ffma2_rn(mr3, __ffma2_rn(a3, dy, dvy), s.jy);
     s.jz = __ffma2_rn(mr3, __ffma2_rn(a3, dz, dvz), s.jz);
-    if (r2nn.x < s.nr2) {
-        s.nr2 = r2nn.x;
-        s.nj = jg0;
-    }
-    if (r2nn.y < s.nr2) {
-        s.nr2 = r2nn.y;
-        s.nj = jg0 + 1;
+    if (STATS) {
+        s.nr2 = fminf(fminf(s.nr2, r2nn.x), r2nn.y);  // which j it was: nn_of_run
+    } else {
+        if (r2nn.x < s.nr2) {
+            s.nr2 = r2nn.x;
+            s.nj = jg0;
+        }
+        if (r2nn.y < s.nr2) {
+            s.nr2 = r2nn.y;
+            s.nj = jg0 + 1;
+        }
     }
     if (NB) {
         const bool hit0 = CHK && self0 ? (p.include_self && s.h2 > 0.f) : (r2n.x < s.h2);
@@ -510,17 +533,31 @@ __device__ __forceinline__ void fold(StateMixedBase &s) {
     s.ax = s.ay = s.az = s.jx = s.jy = s.jz = s.pt = 0.f;
 }
 
-// The nearest neighbour in two steps (FP64 kernels): the pair loop keeps a
-// minimum alone, and after every run of NnRun records it is compared with
-// its value before the run, so the run that first reached the minimum is
-// known.  At the end of the task that run's records are looked through again
-// (nn_scan_run): the same j as a compare and select in every pair term.  A
-// run divides a thread's share of a tile (a multiple of 16 records at 32
-// i-lanes, 4 at 8 i-lanes, any number at 1).
+// The nearest neighbour in two steps (single-call paired kernel, FP64
+// kernels): the pair loop keeps a minimum alone, and after every run of
+// NnRun records it is compared with its value before the run, so the run
+// that first reached the minimum is known.  At the end of the task that
+// run's records are looked through again (nn_of_run, nn_scan_run): the same
+// j as a compare and select in every pair term.  A run divides a thread's
+// share of a tile (a multiple of 16 records at 32 i-lanes, 4 at 8 i-lanes,
+// any number at 1).
 template <int K, int JL, int R, int V> struct NnRun {
     static constexpr int value =
         JL == 1 ? (K == kKernF64 && (R == 2 || (V & (kVarG4 | kVarPot)) != 0) ? 16 : 8) : (JL == 4 ? 4 : 1);
 };
+
+template <int JL, int RUN, bool IDENT>
+__device__ __forceinline__ void nn_of_run(StateMixedP &s, const JPairMixed *jrec) {
+#pragma unroll 1
+    for (int u = 0; u < RUN; ++u) {
+        const int k = s.nk + u * JL;
+        const float2 r2 = pair_nn_r2<IDENT>(s, jrec[k], 2 * k);
+        if (r2.x == s.nr2 || r2.y == s.nr2) {
+            s.nj = 2 * k + (r2.x == s.nr2 ? 0 : 1);
+            return;
+        }
+    }
+}
 
 // Consume one shared-memory tile: this thread's j are kbase + m*JL.
 template <int K, int R, int JL, bool CHK, bool NB, bool IDENT, int V>
@@ -532,47 +569,46 @@ __device__ __forceinline__ void consume_tile(typename StateOf<K>::type (&st)[R],
         constexpr bool ST = (V & kVarStats) != 0;
         const float2 eps2 = dup((float)p.eps2);
         constexpr int kFlushPairs = kFlush / 2;
-        if constexpr (kFlushPairs <= 2) {
-            // Short folds: every one or two pair records go into FP64.
-#pragma unroll 4
-            for (int m = 0; m < per; m += kFlushPairs) {
+        if constexpr (ST) {
+            constexpr int RUN = NnRun<K, JL, R, V>::value;
+            // Unrolled by two runs, 16 records: 65536 x 262144 in 23.07 ms
+            // (one run 23.38, a compare and select per term 23.78).
+#pragma unroll 2
+            for (int m0 = 0; m0 < per; m0 += RUN) {
+                float before[R];
 #pragma unroll
-                for (int u = 0; u < kFlushPairs; ++u) {
-                    if (u == 0 || m + u < per) {
-                        const int k = kbase + (m + u) * JL;
-                        const JPairMixed J = S[k];
+                for (int r = 0; r < R; ++r) before[r] = st[r].nr2;
 #pragma unroll
-                        for (int r = 0; r < R; ++r)
-                            interact_pair<CHK, NB, IDENT, PO, ST>(st[r], J, tb + 2 * k, eps2, p);
+                for (int u = 0; u < RUN; ++u) {
+                    const int k = kbase + (m0 + u) * JL;
+                    const JPairMixed J = S[k];
+#pragma unroll
+                    for (int r = 0; r < R; ++r) interact_pair<CHK, NB, IDENT, PO, ST>(st[r], J, tb + 2 * k, eps2, p);
+                    if (kFlushPairs < RUN && (u + 1) % kFlushPairs == 0) {
+#pragma unroll
+                        for (int r = 0; r < R; ++r) fold(st[r]);
                     }
                 }
 #pragma unroll
-                for (int r = 0; r < R; ++r) fold_any<PO>(st[r]);
+                for (int r = 0; r < R; ++r)
+                    if (st[r].nr2 < before[r]) st[r].nk = tb / 2 + kbase + m0 * JL;
+                if (kFlushPairs >= RUN && ((m0 + RUN) % kFlushPairs == 0 || m0 + RUN >= per)) {
+#pragma unroll
+                    for (int r = 0; r < R; ++r) fold(st[r]);
+                }
             }
             return;
         }
-        // The single-call kernels (error indicators on) unroll by 16
-        // (measured against 2, 4, 8 and 32 on the N = 262144 sweep: 97.6 ms
-        // at 4, 95.1 at 16; 32 spills); the batched and resident kernels,
-        // which hold three lane shapes in one body, by 4 (at 16 they spill).
+        // The batched and resident kernels, which hold three lane shapes in
+        // one body, unroll by 4 (at 16 they spill).
         for (int m0 = 0; m0 < per; m0 += kFlushPairs) {
             const int m1 = min(m0 + kFlushPairs, per);
-            if constexpr (ST) {
-#pragma unroll 16
-                for (int m = m0; m < m1; ++m) {
-                    const int k = kbase + m * JL;
-                    const JPairMixed J = S[k];
+#pragma unroll (PO ? 8 : 4)
+            for (int m = m0; m < m1; ++m) {
+                const int k = kbase + m * JL;
+                const JPairMixed J = S[k];
 #pragma unroll
-                    for (int r = 0; r < R; ++r) interact_pair<CHK, NB, IDENT, PO, ST>(st[r], J, tb + 2 * k, eps2, p);
-                }
-            } else {
-#pragma unroll 4
-                for (int m = m0; m < m1; ++m) {
-                    const int k = kbase + m * JL;
-                    const JPairMixed J = S[k];
-#pragma unroll
-                    for (int r = 0; r < R; ++r) interact_pair<CHK, NB, IDENT, PO, ST>(st[r], J, tb + 2 * k, eps2, p);
-                }
+                for (int r = 0; r < R; ++r) interact_pair<CHK, NB, IDENT, PO, ST>(st[r], J, tb + 2 * k, eps2, p);
             }
 #pragma unroll
             for (int r = 0; r < R; ++r) fold_any<PO>(st[r]);
@@ -857,7 +893,8 @@ __device__ __forceinline__ bool process_task(const ForceParams &p, int itile_idx
     // Records of the last two tiles are still in shared memory, the others
     // are read where they came from.
     constexpr int RUN = NnRun<K, JL, R, V>::value;
-    constexpr bool kRunNn = K == kKernF64 && (V & (kVarG4 | kVarPot)) == 0;
+    constexpr bool kRunNn = (K == kKernMixedP && (V & kVarStats) != 0) ||
+                            (K == kKernF64 && (V & (kVarG4 | kVarPot)) == 0);
     auto records_of = [&](int unit) -> const JRec * {
         const int t2 = (unit * JPU - jb) / T;
         return t2 >= ntiles - 2 ? tiles + ((g0 + t2) & 1) * U - (jb + t2 * T) / JPU : jrec;
@@ -865,6 +902,9 @@ __device__ __forceinline__ bool process_task(const ForceParams &p, int itile_idx
     Partial q[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
+        if constexpr (K == kKernMixedP && kRunNn) {
+            if (st[r].nk >= 0) nn_of_run<JL, RUN, IDENT>(st[r], jrec);
+        }
         if constexpr (K == kKernF64) {
             const int first = jb + kbase;
             // A sum that is not finite: some r^2 overflowed, vanished, or is
@@ -893,7 +933,7 @@ __device__ __forceinline__ bool process_task(const ForceParams &p, int itile_idx
         if (JL > 1) warp_reduce<IL>(q[r]);
     }
     if (H > 1) {
-        if (kRunNn) __syncthreads();  // the tile area was read above
+        if (K == kKernF64 && kRunNn) __syncthreads();  // the tile area was read above
         if (jl == 0) {
 #pragma unroll
             for (int r = 0; r < R; ++r) red[h * itile + islot + r * IL] = q[r];
