@@ -120,6 +120,7 @@ int Engine::open(int device, int nmax_hint) {
     cudaEvent_t *evs[] = {&ev_stage_, &ev_begin_, &ev_pred0_, &ev_pred1_, &ev_force0_, &ev_force1_, &ev_done_};
     for (cudaEvent_t *e : evs) G6_CHECK(cudaEventCreate(e), "event");
     G6_CHECK(cudaEventCreateWithFlags(&ev_ext_, cudaEventDisableTiming), "event");
+    G6_CHECK(prepare_small_force(), "small call kernels");
     stage_cap_ = 16384;
     G6_CHECK(cudaMallocHost(&h_stage_vals_, sizeof(double) * JF_COUNT * stage_cap_), "pinned stage");
     G6_CHECK(cudaMallocHost(&h_stage_addr_, sizeof(int) * stage_cap_), "pinned stage");
@@ -704,6 +705,7 @@ int Engine::launch_call() {
     }
     unsigned *status = status2 + call_parity_;
     pred_timed_ = false;
+    bool one_launch = false;
     const bool staged = small && n_staged_ > 0;
     bool need_pred;
     if (call_f64_) {
@@ -745,12 +747,21 @@ int Engine::launch_call() {
         if (call_g4_) memcpy(sc.ieps2, h_ieps2_, sizeof(double) * ni);
         stats_.h2d_bytes += (long long)sizeof(SmallCall);
         n_staged_ = 0;
-        if (timed_) G6_CHECK(cudaEventRecord(ev_pred0_, stream_), "event");
-        launch_small_call(stream_, km, sc, d_jraw_, d_jindex_, jrec, d_irec_, d_ieps2_, status2);
-        G6_CHECK(cudaGetLastError(), "small call launch");
-        stats_.launches++;
-        if (timed_) G6_CHECK(cudaEventRecord(ev_pred1_, stream_), "event");
-        pred_timed_ = need_pred;
+        // FP64 force calls go further: updates, prediction and forces are one
+        // launch (launch_small_force below) when each CTA's j-range fits its
+        // shared memory.
+        ForceParams probe{};
+        probe.nj_pad = nj_pad;
+        one_launch = km == kKernF64 && need_pred && ni > 0 && !call_pot_ && !call_split_ && override_.il <= 0 &&
+                     small_force_fits(choose_config(km, ni, nj_pad, num_sms_, call_nb_), probe);
+        if (!one_launch) {
+            if (timed_) G6_CHECK(cudaEventRecord(ev_pred0_, stream_), "event");
+            launch_small_call(stream_, km, sc, d_jraw_, d_jindex_, jrec, d_irec_, d_ieps2_, status2);
+            G6_CHECK(cudaGetLastError(), "small call launch");
+            stats_.launches++;
+            if (timed_) G6_CHECK(cudaEventRecord(ev_pred1_, stream_), "event");
+            pred_timed_ = need_pred;
+        }
         if (need_pred) {
             stats_.predictions++;
             mark_predicted(nj, km);
@@ -821,8 +832,12 @@ int Engine::launch_call() {
         p.out_q = call_refine_ ? d_q_ : nullptr;
         if (call_nb_) G6_CHECK(cudaMemsetAsync(d_nb_count_, 0, sizeof(int) * ni, stream_), "memset");
         if (timed_) G6_CHECK(cudaEventRecord(ev_force0_, stream_), "event");
-        G6_CHECK(launch_force(stream_, km, cfg, p, n_nonident_ == 0 && !call_g4_, call_nb_, call_g4_, pot_k),
-                 "force launch");
+        if (one_launch)
+            G6_CHECK(launch_small_force(stream_, cfg, p, small_call_, d_jraw_, d_jindex_, status2,
+                                        n_nonident_ == 0 && !call_g4_, call_nb_), "force launch");
+        else
+            G6_CHECK(launch_force(stream_, km, cfg, p, n_nonident_ == 0 && !call_g4_, call_nb_, call_g4_, pot_k),
+                     "force launch");
         if (timed_) G6_CHECK(cudaEventRecord(ev_force1_, stream_), "event");
         stats_.launches += 1;
         if (call_refine_) {

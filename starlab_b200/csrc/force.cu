@@ -65,6 +65,30 @@ __global__ void __launch_bounds__(256, MinBlocks<K, R>::value) force_kernel(cons
     process_task<K, IL, R, NB, IDENT, V>(p, blockIdx.x, blockIdx.y, smem, gt);
 }
 
+// A small FP64 call in one launch: its staged updates to the raw j-state,
+// the prediction of each CTA's j-range, the forces (process_task's JFromCall
+// form).  As two launches (updates and prediction, then forces) a block of
+// 61 against 40009 j took 14.2 + 30.0 us on the device, one of 24 against
+// 1024 10.5 + 9.5; as one 23.3 and 10.5.
+template <int IL, bool NB, bool IDENT, int V>
+__global__ void __launch_bounds__(256, 1)
+    small_force_kernel(const __grid_constant__ SmallCall param, ForceParams p, double *jraw, int *jindex,
+                       unsigned *status2) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ int s_addr[kSmallMax];
+    const SmallCall &sc = param_as_memory(param);
+    if (threadIdx.x < sc.n_upd) s_addr[threadIdx.x] = sc.addr[threadIdx.x];
+    const int cta = blockIdx.x + gridDim.x * blockIdx.y;
+    if (cta == 0 && threadIdx.x == 0) status2[sc.parity ^ 1] = 0u;
+    store_updates(sc, cta, gridDim.x * gridDim.y, jraw, jindex);
+    p.irec = sc.irec;
+    p.ieps2 = sc.g4 ? sc.ieps2 : nullptr;
+    __syncthreads();
+    int gt = 0;
+    process_task<kKernF64, IL, 1, NB, IDENT, V, JFromCall>(p, blockIdx.x, blockIdx.y, smem, gt,
+                                                           JFromCall{&sc, jraw, jindex, s_addr});
+}
+
 // Many calls in one launch: items[k] is one call (its own j-memory,
 // i-records, softening, fixed-point scale and outputs); its tasks are
 // n_itiles(k) x nsplit(k), numbered from task0[k].  Persistent form: CTAs
@@ -314,18 +338,10 @@ cudaError_t launch_force_batch(cudaStream_t s, int kmode, const ForceConfig &cfg
     return e;
 }
 
-cudaError_t launch_force(cudaStream_t s, int kmode, const ForceConfig &cfg, ForceParams p,
-                         bool ident, bool nb, bool g4, bool pot) {
-    if (g4 && (kmode != kKernF64 || !p.ieps2)) return cudaErrorInvalidValue;
-    if (pot && (g4 || nb || cfg.r != 1 || kmode == kKernMixedDS)) return cudaErrorInvalidValue;
-    const int T = tile_size(kmode);
-    const int ntiles = p.nj_pad / T;
-    if (p.ni <= 0) return cudaSuccess;
-    if (cfg.jper > 0) {
-        if (cfg.jper % T) return cudaErrorInvalidValue;
-        p.jper = cfg.jper;
-        p.nsplit = std::max(1, (p.nj_pad + cfg.jper - 1) / cfg.jper);
-    } else if (ntiles <= 0) {
+// Fills jper, nsplit and H of p as launch_force does, and returns its i-tile.
+static int plan_call(int kmode, const ForceConfig &cfg, ForceParams &p) {
+    const int T = tile_size(kmode), ntiles = p.nj_pad / T;
+    if (ntiles <= 0) {
         p.jper = T;
         p.nsplit = 1;
     } else {
@@ -334,8 +350,66 @@ cudaError_t launch_force(cudaStream_t s, int kmode, const ForceConfig &cfg, Forc
         p.nsplit = (ntiles + per_split_tiles - 1) / per_split_tiles;
     }
     p.H = cfg.H;
-    const int G = cfg.warps / cfg.H;
-    const int itile = G * cfg.il * cfg.r;
+    return cfg.warps / cfg.H * cfg.il * cfg.r;
+}
+
+using SmallFn = void (*)(const SmallCall, ForceParams, double *, int *, unsigned *);
+
+template <int IL>
+static SmallFn pick_small(bool nb, bool ident, bool g4) {
+    constexpr int V = kVarUnroll4;
+    if (g4) return nb ? small_force_kernel<IL, true, false, kVarG4> : small_force_kernel<IL, false, false, kVarG4>;
+    if (nb) return ident ? small_force_kernel<IL, true, true, V> : small_force_kernel<IL, true, false, V>;
+    return ident ? small_force_kernel<IL, false, true, V> : small_force_kernel<IL, false, false, V>;
+}
+
+static SmallFn pick_small(int il, bool nb, bool ident, bool g4) {
+    return il == 32 ? pick_small<32>(nb, ident, g4) : il == 8 ? pick_small<8>(nb, ident, g4)
+                                                              : pick_small<1>(nb, ident, g4);
+}
+
+static size_t small_smem_bytes(const ForceConfig &cfg, const ForceParams &p, int itile) {
+    const size_t j = (size_t)p.jper * sizeof(JRecF64);
+    const size_t red = std::max((size_t)cfg.H * itile, (size_t)16 * cfg.warps) * sizeof(Partial);
+    return 128 + std::max(j, red);
+}
+
+bool small_force_fits(const ForceConfig &cfg, ForceParams p) {
+    const int itile = plan_call(kKernF64, cfg, p);
+    return cfg.r == 1 && cfg.H > 1 && p.nj_pad > 0 && small_smem_bytes(cfg, p, itile) <= kSmallSmemMax;
+}
+
+cudaError_t prepare_small_force() {
+    for (int il : {32, 8, 1})
+        for (int v = 0; v < 6; ++v) {
+            const cudaError_t e = cudaFuncSetAttribute(pick_small(il, v & 1, v & 2, v >= 4),
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmemMax);
+            if (e != cudaSuccess) return e;
+        }
+    return cudaSuccess;
+}
+
+cudaError_t launch_small_force(cudaStream_t s, const ForceConfig &cfg, ForceParams p, const SmallCall &sc,
+                               double *jraw, int *jindex, unsigned *status2, bool ident, bool nb) {
+    const int itile = plan_call(kKernF64, cfg, p);
+    const dim3 grid((p.ni + itile - 1) / itile, p.nsplit);
+    pick_small(cfg.il, nb, ident, sc.g4 != 0)<<<grid, 32 * cfg.warps, small_smem_bytes(cfg, p, itile), s>>>(
+        sc, p, jraw, jindex, status2);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_force(cudaStream_t s, int kmode, const ForceConfig &cfg, ForceParams p,
+                         bool ident, bool nb, bool g4, bool pot) {
+    if (g4 && (kmode != kKernF64 || !p.ieps2)) return cudaErrorInvalidValue;
+    if (pot && (g4 || nb || cfg.r != 1 || kmode == kKernMixedDS)) return cudaErrorInvalidValue;
+    const int T = tile_size(kmode);
+    if (p.ni <= 0) return cudaSuccess;
+    const int itile = plan_call(kmode, cfg, p);
+    if (cfg.jper > 0) {
+        if (cfg.jper % T) return cudaErrorInvalidValue;
+        p.jper = cfg.jper;
+        p.nsplit = std::max(1, (p.nj_pad + cfg.jper - 1) / cfg.jper);
+    }
     dim3 grid((p.ni + itile - 1) / itile, p.nsplit);
     dim3 block(32 * cfg.warps);
     KernelFn fn = pot ? (kmode == kKernF64 ? pick_pot<kKernF64>(cfg.il, ident) : pick_pot<kKernMixedP>(cfg.il, ident))

@@ -8,6 +8,7 @@
 #include <cfloat>
 #include "common.cuh"
 #include "kernels.h"
+#include "predict_device.cuh"
 
 namespace g6 {
 
@@ -867,14 +868,83 @@ template <int K, int R> struct MinBlocks {
     static constexpr int value = R >= 4 ? 1 : 2;
 };
 
+// Where a task's j come from: predicted records in device memory, copied
+// tile by tile,
+struct JRecords {
+    static constexpr bool kInPlace = false;
+};
+// or a small FP64 call's raw j-state and updates, predicted by the CTA that
+// needs them: its whole j-range, into shared memory in one pass (so the
+// loads' latency is paid once) and, by the first i-tile's CTAs, into the
+// record array too, which then holds the prediction for later calls.
+struct JFromCall {
+    static constexpr bool kInPlace = true;
+    const SmallCall *sc;
+    double *jraw;
+    int *jindex;
+    int *s_addr;  // [kSmallMax] in shared memory
+};
+
+__device__ __forceinline__ void predict_range(const JFromCall &src, const ForceParams &p, int jb, int n, bool store,
+                                              bool last, JRecF64 *tiles) {
+    const SmallCall &sc = *src.sc;
+    JRecF64 *out = static_cast<JRecF64 *>(const_cast<void *>(p.jrec));
+    constexpr int B = 2;  // records per thread whose loads are issued together
+    for (int r0 = threadIdx.x; r0 < n; r0 += B * blockDim.x) {
+        double raw[B][JF_K18];
+        int id[B];
+#pragma unroll
+        for (int u = 0; u < B; ++u) {
+            const int j = jb + r0 + u * (int)blockDim.x;
+            if (r0 + u * (int)blockDim.x < n && j < sc.nj) {
+#pragma unroll
+                for (int f = 0; f < JF_K18; ++f) raw[u][f] = src.jraw[(size_t)f * sc.cap + j];
+                id[u] = src.jindex[j];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < B; ++u) {
+            const int r = r0 + u * (int)blockDim.x, j = jb + r;
+            if (r >= n) break;
+            JRecF64 rec;
+            if (j < sc.nj) {
+                // an updated particle's raw state is being rewritten: its
+                // values are the update's
+                const int k = find_update(src.s_addr, sc.n_upd, j);
+                double xp[3], vp[3], m;
+                if (k >= 0) {
+                    predict_vals(sc.vals[k], sc.ti, xp, vp, m);
+                    id[u] = sc.index[k];
+                } else {
+                    predict_vals(raw[u], sc.ti, xp, vp, m);
+                }
+                rec.pos = make_double4(xp[0], xp[1], xp[2], m);
+                rec.vel = make_double4(vp[0], vp[1], vp[2], (double)id[u]);
+            } else {
+                rec.pos = make_double4(kDummyPos, kDummyPos, kDummyPos, 0.0);
+                rec.vel = make_double4(0.0, 0.0, 0.0, -1.0);
+            }
+            tiles[r] = rec;
+            if (store) out[j] = rec;
+        }
+    }
+    // the record array's padding may be wider than this kernel's tiles
+    if (store && last) {
+        JRecF64 rec;
+        rec.pos = make_double4(kDummyPos, kDummyPos, kDummyPos, 0.0);
+        rec.vel = make_double4(0.0, 0.0, 0.0, -1.0);
+        for (int j = p.nj_pad + threadIdx.x; j < sc.nj_pad; j += blockDim.x) out[j] = rec;
+    }
+}
+
 // One task: the i-tile `itile_idx` of item p against its j-split `split`.
 // Shared memory holds the two mbarriers (initialised by the caller) and the
 // tile ring; `gt` counts the tiles this CTA consumed before (it sets the
 // ring stage and the mbarrier phase, so a persistent CTA can run many
 // tasks back to back).
-template <int K, int IL, int R, bool NB, bool IDENT, int V>
+template <int K, int IL, int R, bool NB, bool IDENT, int V, class Src = JRecords>
 __device__ __forceinline__ bool process_task(const ForceParams &p, int itile_idx, int split, unsigned char *smem,
-                                             int &gt) {
+                                             int &gt, const Src &src = Src{}) {
     using Tr = Traits<K>;
     using JRec = typename Tr::JRec;
     using State = typename StateOf<K>::type;
@@ -917,28 +987,9 @@ __device__ __forceinline__ bool process_task(const ForceParams &p, int itile_idx
     const JRec *jrec = reinterpret_cast<const JRec *>(p.jrec);
     const int g0 = gt;
 
-    // The previous task's epilogue may still read the tile area.
-    __syncthreads();
-    if (threadIdx.x == 0 && ntiles > 0) {
-        const int b = g0 & 1;
-        mbar_arrive_expect_tx(&bars[b], kTileBytes);
-        bulk_g2s(tiles + b * U, jrec + jb / JPU, kTileBytes, &bars[b]);
-    }
-
     const int per = U / (H * JL);
     const int kbase = h * (U / H) + jl;
-    bool ok = true;
-    int t = 0;
-    for (; t < ntiles; ++t) {
-        const int gg = g0 + t;
-        const int b = gg & 1;
-        if (threadIdx.x == 0 && t + 1 < ntiles) {
-            mbar_arrive_expect_tx(&bars[b ^ 1], kTileBytes);
-            bulk_g2s(tiles + (b ^ 1) * U, jrec + (jb + (t + 1) * T) / JPU, kTileBytes, &bars[b ^ 1]);
-        }
-        const bool arrived = mbar_wait_bounded(&bars[b], (gg >> 1) & 1, kWaitLimitNs);
-        const JRec *S = tiles + b * U;
-        const int tb = jb + t * T;
+    auto consume = [&](const JRec *S, int tb) {
         bool chk = true;
         if (IDENT) {
             bool mine = false;
@@ -950,11 +1001,37 @@ __device__ __forceinline__ bool process_task(const ForceParams &p, int itile_idx
             consume_tile<K, R, JL, true, NB, IDENT, V>(st, S, kbase, per, tb, p);
         else
             consume_tile<K, R, JL, false, NB, IDENT, V>(st, S, kbase, per, tb, p);
-        // The barrier that frees the tile buffer for the next copy also makes
-        // a timed-out wait (on any thread) the whole CTA's decision.
-        if (__syncthreads_or(!arrived)) {
-            ok = false;
-            break;
+    };
+    bool ok = true;
+    int t = 0;
+    if constexpr (Src::kInPlace) {
+        predict_range(src, p, jb, ntiles * T, itile_idx == 0, je == p.nj_pad, tiles);
+        __syncthreads();
+        for (; t < ntiles; ++t) consume(tiles + t * U, jb + t * T);
+    } else {
+        // The previous task's epilogue may still read the tile area.
+        __syncthreads();
+        if (threadIdx.x == 0 && ntiles > 0) {
+            const int b = g0 & 1;
+            mbar_arrive_expect_tx(&bars[b], kTileBytes);
+            bulk_g2s(tiles + b * U, jrec + jb / JPU, kTileBytes, &bars[b]);
+        }
+
+        for (; t < ntiles; ++t) {
+            const int gg = g0 + t;
+            const int b = gg & 1;
+            if (threadIdx.x == 0 && t + 1 < ntiles) {
+                mbar_arrive_expect_tx(&bars[b ^ 1], kTileBytes);
+                bulk_g2s(tiles + (b ^ 1) * U, jrec + (jb + (t + 1) * T) / JPU, kTileBytes, &bars[b ^ 1]);
+            }
+            const bool arrived = mbar_wait_bounded(&bars[b], (gg >> 1) & 1, kWaitLimitNs);
+            consume(tiles + b * U, jb + t * T);
+            // The barrier that frees the tile buffer for the next copy also makes
+            // a timed-out wait (on any thread) the whole CTA's decision.
+            if (__syncthreads_or(!arrived)) {
+                ok = false;
+                break;
+            }
         }
     }
     gt = g0 + ntiles;
@@ -973,12 +1050,15 @@ __device__ __forceinline__ bool process_task(const ForceParams &p, int itile_idx
     }
 
     // ---- epilogue: lanes -> warps -> (output | split partial)
-    // Records of the last two tiles are still in shared memory, the others
-    // are read where they came from.
+    // Records of the last two tiles are still in shared memory (all of them
+    // when they were predicted here), the others are read where they came
+    // from.
     constexpr int RUN = NnRun<K, JL, R, V>::value;
     constexpr bool kRunNn = (K == kKernMixedP && (V & kVarStats) != 0) ||
                             (K == kKernF64 && (V & (kVarG4 | kVarPot)) == 0);
+    const JRec *all = Src::kInPlace ? tiles - jb / JPU : jrec;
     auto records_of = [&](int unit) -> const JRec * {
+        if (Src::kInPlace) return all;
         const int t2 = (unit * JPU - jb) / T;
         return t2 >= ntiles - 2 ? tiles + ((g0 + t2) & 1) * U - (jb + t2 * T) / JPU : jrec;
     };
@@ -986,7 +1066,7 @@ __device__ __forceinline__ bool process_task(const ForceParams &p, int itile_idx
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         if constexpr (K == kKernMixedP && kRunNn) {
-            if (st[r].nk >= 0) nn_of_run<JL, RUN, IDENT>(st[r], jrec);
+            if (st[r].nk >= 0) nn_of_run<JL, RUN, IDENT>(st[r], all);
         }
         if constexpr (K == kKernF64) {
             const int first = jb + kbase;
@@ -999,14 +1079,14 @@ __device__ __forceinline__ bool process_task(const ForceParams &p, int itile_idx
 #pragma unroll 1
                     for (int m = 0; m < per; ++m) {
                         const int jg = first + t2 * T + m * JL;
-                        interact_any<true, IDENT, (V & kVarG4) != 0, (V & kVarPot) != 0>(st[r], jrec[jg].pos,
-                                                                                        jrec[jg].vel, jg);
+                        interact_any<true, IDENT, (V & kVarG4) != 0, (V & kVarPot) != 0>(st[r], all[jg].pos,
+                                                                                        all[jg].vel, jg);
                     }
             }
             if constexpr (kRunNn) {
                 if (st[r].ntie) {
 #pragma unroll 1
-                    for (int t2 = 0; t2 < ntiles; ++t2) nn_scan<JL, IDENT>(st[r], jrec, first + t2 * T, per);
+                    for (int t2 = 0; t2 < ntiles; ++t2) nn_scan<JL, IDENT>(st[r], all, first + t2 * T, per);
                 } else if (st[r].nk >= 0) {
                     nn_scan_run<JL, RUN, IDENT>(st[r], records_of(st[r].nk), st[r].nk);
                 }
@@ -1016,7 +1096,7 @@ __device__ __forceinline__ bool process_task(const ForceParams &p, int itile_idx
         if (JL > 1) warp_reduce<IL>(q[r]);
     }
     if (H > 1) {
-        if (K == kKernF64 && kRunNn) __syncthreads();  // the tile area was read above
+        if (Src::kInPlace || (K == kKernF64 && kRunNn)) __syncthreads();  // the tile area was read above
         if (jl == 0) {
 #pragma unroll
             for (int r = 0; r < R; ++r) red[h * itile + islot + r * IL] = q[r];

@@ -159,6 +159,15 @@ ForceConfig choose_config(int kmode, int ni, int nj_pad, int num_sms, bool nb);
 // layout, cfg.r == 1, no neighbour lists.
 cudaError_t launch_force(cudaStream_t s, int kmode, const ForceConfig &cfg, ForceParams p,
                          bool ident, bool nb, bool g4 = false, bool pot = false);
+// A small FP64 call as one launch: updates, prediction and forces (no
+// irec, ieps2 or records read; the records are written).  Fits when a CTA's
+// j-range fits into shared memory.  prepare: once per device before the
+// first launch.
+constexpr int kSmallSmemMax = 200 * 1024;
+bool small_force_fits(const ForceConfig &cfg, ForceParams p);
+cudaError_t prepare_small_force();
+cudaError_t launch_small_force(cudaStream_t s, const ForceConfig &cfg, ForceParams p, const SmallCall &sc,
+                               double *jraw, int *jindex, unsigned *status2, bool ident, bool nb);
 size_t partial_bytes(const ForceConfig &cfg, int ni);
 // Partial-sum bytes of a launch whose splits hold jper j each (keep_partials).
 size_t partial_bytes_fixed(int jper, int nj_pad, int ni);

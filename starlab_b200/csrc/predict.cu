@@ -119,53 +119,13 @@ __global__ void irec_from_j_kernel(const double *__restrict__ jraw, const int *_
 
 // ---- small calls: updates + prediction + i-records in one launch
 
-__device__ __forceinline__ void predict_vals(const double *v17, double ti, double xp[3], double vp[3], double &m) {
-    const double dt = ti - v17[JF_T];
-    m = v17[JF_M];
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-        const double x = v17[JF_X + c], v = v17[JF_V + c], a2 = v17[JF_A2 + c], j6 = v17[JF_J6 + c];
-        xp[c] = x + dt * (v + dt * (a2 + dt * j6));
-        vp[c] = v + dt * (2.0 * a2 + dt * (3.0 * j6));
-    }
-}
-
-// Position of address j in the ascending update list, or -1.
-__device__ __forceinline__ int find_update(const int *addr, int n, int j) {
-    int lo = 0, hi = n - 1;
-    while (lo <= hi) {
-        const int mid = (lo + hi) >> 1;
-        const int a = addr[mid];
-        if (a == j) return mid;
-        if (a < j) lo = mid + 1; else hi = mid - 1;
-    }
-    return -1;
-}
-
-// Predicted j (or a dummy beyond nj): the update's values when j is being
-// updated (its raw state is rewritten by another thread of this launch),
-// the raw j-state otherwise.
-__device__ __forceinline__ bool small_pred(const SmallCall &sc, const int *s_addr, const double *jraw,
-                                           const int *jindex, int j, double xp[3], double vp[3], double &m,
-                                           int &id) {
-    if (j >= sc.nj) return false;
-    const int s = find_update(s_addr, sc.n_upd, j);
-    if (s >= 0) {
-        predict_vals(sc.vals[s], sc.ti, xp, vp, m);
-        id = sc.index[s];
-    } else {
-        predict_one(jraw, sc.cap, j, sc.ti, xp, vp, m);
-        id = jindex[j];
-    }
-    return true;
-}
-
 template <int KM>
-__global__ void __launch_bounds__(256) small_call_kernel(const __grid_constant__ SmallCall sc,
-                                                         double *__restrict__ jraw, int *__restrict__ jindex,
+__global__ void __launch_bounds__(256) small_call_kernel(const __grid_constant__ SmallCall param,
+                                                         double *jraw, int *jindex,
                                                          void *__restrict__ jrec, IRec *__restrict__ irec,
                                                          double *__restrict__ ieps2, unsigned *__restrict__ status2) {
     __shared__ int s_addr[kSmallMax];
+    const SmallCall &sc = param_as_memory(param);
     const int tid = threadIdx.x;
     if (tid < sc.n_upd) s_addr[tid] = sc.addr[tid];
     if (blockIdx.x == 0) {
@@ -174,13 +134,8 @@ __global__ void __launch_bounds__(256) small_call_kernel(const __grid_constant__
             if (sc.g4) ieps2[tid] = sc.ieps2[tid];
         }
         if (tid == 0) status2[sc.parity ^ 1] = 0u;
-        if (tid < sc.n_upd) {  // persist the updates (no thread of this launch reads these addresses' raw state)
-            const int a = sc.addr[tid];
-#pragma unroll
-            for (int f = 0; f < JF_COUNT; ++f) jraw[(size_t)f * sc.cap + a] = sc.vals[tid][f];
-            jindex[a] = sc.index[tid];
-        }
     }
+    store_updates(sc, blockIdx.x, gridDim.x, jraw, jindex);
     __syncthreads();
     if (!sc.predict) return;
     const int q = blockIdx.x * blockDim.x + tid;
