@@ -108,3 +108,19 @@ def test_batched_and_per_cluster_agree_and_conserve_energy():
         assert np.max(np.abs(a["x"] - b["x"])) < 1e-4
     e1.close()
     e2.close()
+
+
+@pytest.mark.parametrize("sizes", [(1, 2, 255), (256, 257, 1), (1000, 31, 4097)])
+def test_get_returns_the_clusters_own_rows(sizes):
+    """The state read back at the start is the one set, particle by particle
+    (odd sizes: the rows are packed for one cluster at a time)."""
+    from starlab_b200.ensemble import Ensemble
+    cl = [c[:3] for c in clusters(sizes, 40)]
+    ens = Ensemble([c[0] for c in cl], [c[1] for c in cl], [c[2] for c in cl], 1e-4)
+    ens.start()
+    for c, (m, x, v) in enumerate(cl):
+        g = ens.get(c)
+        assert np.array_equal(g["m"], m) and np.array_equal(g["x"], x) and np.array_equal(g["v"], v)
+        assert np.all(g["t"] == 0.0) and np.all(g["dt"] > 0.0)
+        assert np.any(g["acc"][0] != 0.0) == (len(m) > 1)
+    ens.close()
