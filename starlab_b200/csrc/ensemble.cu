@@ -761,6 +761,7 @@ int Ensemble::setup() {
     // iteration against 225.
     d_.cfg.nsplit = 592;
     d_.cfg.min_tiles = min_tiles_;
+    d_.cfg.fine_ni = kEnsFineNi;
     ctas_ = batch_ctas(kmode_, d_.cfg, num_sms_);
     ECHK(cudaMemcpyAsync((void *)d_.off, off_.data(), sizeof(int) * (nc_ + 1), cudaMemcpyHostToDevice, stream_), "copy");
     ECHK(cudaMemcpyAsync((void *)d_.n, n_.data(), sizeof(int) * nc_, cudaMemcpyHostToDevice, stream_), "copy");
