@@ -68,8 +68,8 @@ struct StateF64 {
     double eps2;  // softening: the call's, or (GRAPE-4 variant) this i's
     double Ax, Ay, Az, Jx, Jy, Jz, Pt;  // acc, jerk x 3 sqrt(3), pot x sqrt(3): see inv_dist_s3
     unsigned nhi;  // smallest upper word of r^2 so far
-    int nk;        // first j of the run that first reached it (-1: none)
-    bool ntie;     // another run reached the same upper word
+    int nk, nk2;   // first j of the run that first reached it and of a second one that did (-1: none)
+    bool ntie;     // a third run reached it
     double nr2;
     int nj, idx, i;
 };
@@ -114,7 +114,7 @@ __device__ __forceinline__ void load_i(StateF64 &s, const IRec &q, const ForcePa
     s.eps2 = p.eps2;
     s.Ax = s.Ay = s.Az = s.Jx = s.Jy = s.Jz = s.Pt = 0.0;
     s.nhi = kHiInf;
-    s.nk = -1;
+    s.nk = s.nk2 = -1;
     s.ntie = false;
     s.nr2 = DBL_MAX;
     s.nj = -1;
@@ -294,9 +294,9 @@ __device__ __forceinline__ unsigned interact(StateF64 &s, const JRecF64 &J, int 
     return hi;
 }
 
-// Nearest neighbour of the FP64 kernels: the j of [j0, j0 + n JL) in steps
-// of JL (addresses) with the smallest unsoftened r^2, the first on a tie.
-// Of a run, up to eight records are loaded before the first is used.
+// Nearest neighbour of the FP64 kernels: of a run of RUN j from j0 in steps
+// of JL (addresses), the one with the smallest unsoftened r^2, the first on
+// a tie.  Up to eight records are loaded before the first is used.
 template <int JL, bool IDENT>
 __device__ __forceinline__ void nn_scan_one(StateF64 &s, const double4 &pos, double w, int jg) {
     const double r2 = r2_f64(pos.x - s.x, pos.y - s.y, pos.z - s.z);
@@ -322,12 +322,6 @@ __device__ __forceinline__ void nn_scan_run(StateF64 &s, const JRecF64 *src, int
 #pragma unroll
         for (int u = 0; u < B; ++u) nn_scan_one<JL, IDENT>(s, pos[u], w[u], j0 + (b + u) * JL);
     }
-}
-
-template <int JL, bool IDENT>
-__device__ __forceinline__ void nn_scan(StateF64 &s, const JRecF64 *jrec, int j0, int n) {
-#pragma unroll 1
-    for (int u = 0; u < n; ++u) nn_scan_one<JL, IDENT>(s, jrec[j0 + u * JL].pos, jrec[j0 + u * JL].vel.w, j0 + u * JL);
 }
 
 // ---- paired layout: one FP32x2 instruction evaluates i against two j.
@@ -636,9 +630,11 @@ __device__ __forceinline__ void consume_tile(typename StateOf<K>::type (&st)[R],
                     if (lo[r] < st[r].nhi) {
                         st[r].nhi = lo[r];
                         st[r].nk = tb + kbase + m0 * JL;
+                        st[r].nk2 = -1;
                         st[r].ntie = false;
                     } else if (lo[r] == st[r].nhi) {
-                        st[r].ntie = true;
+                        st[r].ntie = st[r].nk2 >= 0;
+                        st[r].nk2 = st[r].nk2 >= 0 ? st[r].nk2 : tb + kbase + m0 * JL;
                     }
                 }
             }
@@ -1086,9 +1082,13 @@ __device__ __forceinline__ bool process_task(const ForceParams &p, int itile_idx
             if constexpr (kRunNn) {
                 if (st[r].ntie) {
 #pragma unroll 1
-                    for (int t2 = 0; t2 < ntiles; ++t2) nn_scan<JL, IDENT>(st[r], all, first + t2 * T, per);
+                    for (int t2 = 0; t2 < ntiles; ++t2)
+#pragma unroll 1
+                        for (int m = 0; m < per; m += RUN) nn_scan_run<JL, RUN, IDENT>(st[r], all, first + t2 * T + m * JL);
                 } else if (st[r].nk >= 0) {
-                    nn_scan_run<JL, RUN, IDENT>(st[r], records_of(st[r].nk), st[r].nk);
+#pragma unroll 1
+                    for (int k = st[r].nk; k >= 0; k = k == st[r].nk ? st[r].nk2 : -1)
+                        nn_scan_run<JL, RUN, IDENT>(st[r], records_of(k), k);
                 }
             }
         }
