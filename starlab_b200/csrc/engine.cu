@@ -793,7 +793,9 @@ int Engine::launch_call() {
                 stats_.h2d_bytes += (long long)sizeof(double) * ni;
             }
         }
-        ForceConfig cfg = override_.il > 0 ? override_ : choose_config(km, ni, nj_pad, num_sms_, call_nb_);
+        ForceConfig cfg = override_.il > 0 ? override_
+                          : call_split_ ? fill_config(km, ni, nj_pad, num_sms_)
+                                        : choose_config(km, ni, nj_pad, num_sms_, call_nb_);
         // Potential-only kernel (one i per thread) for the paired mixed and
         // FP64 layouts; the scalar mixed layout runs its full kernel.
         const bool pot_k = call_pot_ && km != kKernMixedDS;

@@ -234,8 +234,11 @@ size_t partial_bytes_fixed(int jper, int nj_pad, int ni) {
     return (size_t)nsplit * ni * sizeof(Partial);
 }
 
-ForceConfig choose_config(int kmode, int ni, int nj_pad, int num_sms, bool nb) {
-    (void)nb;
+// The shape from ni, the splits from a fill rule: blocks of up to 64 i (the
+// i-lane shapes, and the one-launch kernel with its one CTA per SM), the
+// scalar mixed layout, and j-split calls, whose sums must not depend on the
+// size of a rank's slice.
+ForceConfig fill_config(int kmode, int ni, int nj_pad, int num_sms) {
     ForceConfig c;
     c.warps = kMaxWarps;
     c.il = ni >= 32 ? 32 : (ni > 1 ? 8 : 1);
@@ -286,6 +289,81 @@ ForceConfig choose_config(int kmode, int ni, int nj_pad, int num_sms, bool nb) {
     }
     c.nsplit = best_split;
     return c;
+}
+
+// Predicted time (us) of a call's force kernel for a launch shape: fitted to
+// 8000 measured launches (ni 65 to 20096, nj 1024 to 262144, every r and H,
+// up to 24 CTAs per SM).  80 % of the FP64 times lie within -10 and +6 % of
+// it, of the mixed ones within 3 %; the shape it picks is on average 0.4 %
+// (mixed 0.7 %) slower than the best one measured, at worst 5 %.  Filling
+// the SMs' slots with whole waves instead -- which takes a full wave however
+// little work its CTAs then have -- was up to 1.7 times slower than the best
+// (kernel alone: mixed 2048 x 20096 0.129 against 0.075 ms, FP64 2048 x 20096
+// 0.131 against 0.111, 1024 x 4096 0.027 against 0.021).
+//   step   j-steps (records) of the two warps of one CTA on a scheduler
+//   k      CTAs the busiest SM runs, two at a time; an odd last one is alone.
+//          A grid of up to one CTA per SM is counted as two on some: launched
+//          back to back it is spread evenly, in calls it was not (2000 x
+//          262144 in 126 CTAs 1.44 ms a call, in 296 1.40).
+struct ShapeCost {
+    double base, step, alone, cta, tile, round, level;
+};
+constexpr ShapeCost kCostF64{6.3, 0.0427, 0.0034, 2.15, 0.082, 0.96, 0.90};
+constexpr ShapeCost kCostMixed{12.5, 0.0512, 0.0033, 0.0, 0.224, 1.53, 1.10};
+
+static double shape_cost(const ShapeCost &q, int kmode, const ForceConfig &c, int ni, int ntiles, int num_sms) {
+    const int itile = c.warps / c.H * c.il * c.r;
+    const int n_itiles = (ni + itile - 1) / itile;
+    const int per = (ntiles + c.nsplit - 1) / c.nsplit;
+    const int k = std::max(2, (int)(((long long)n_itiles * c.nsplit + num_sms - 1) / num_sms));
+    const double step = (double)per * (units_per_tile(kmode) / c.H) * 2 * c.r;
+    double t = q.base + q.step * k * step + q.cta * k + q.tile * per * ((k + 1) / 2);
+    if (k & 1) t += q.alone * step;
+    if (c.nsplit > 1) {  // the fold: fold_splits' segments, rounds of four loads, pairwise levels
+        int it2 = 1, segs = 1;
+        while (it2 < itile) it2 <<= 1;
+        for (; 2 * segs * it2 <= 32 * c.warps && 8 * segs < c.nsplit; segs <<= 1) t += q.level;
+        t += q.round * ((c.nsplit + segs - 1) / segs) * 0.25 * ((itile + 32 * c.warps - 1) / (32 * c.warps));
+    }
+    return t;
+}
+
+ForceConfig choose_config(int kmode, int ni, int nj_pad, int num_sms, bool nb) {
+    (void)nb;
+    const ForceConfig fill = fill_config(kmode, ni, nj_pad, num_sms);
+    const int ntiles = nj_pad / tile_size(kmode);
+    if (ni <= 64 || ntiles <= 1 || kmode == kKernMixedDS) return fill;
+    const ShapeCost &q = kmode == kKernF64 ? kCostF64 : kCostMixed;
+    ForceConfig best = fill;
+    // the whole waves stay unless 4 % or more is expected: their last wave is
+    // full, which a grid of a few long CTAs does not always achieve
+    double least = 0.96 * shape_cost(q, kmode, fill, ni, ntiles, num_sms);
+    for (int r = 1; r <= (kmode == kKernF64 ? 2 : 1); ++r)
+        for (int H = 1; H <= fill.warps; H *= 2) {
+            // The mixed mode sums 64 terms in FP32: with H of 1, 2 or 4 the
+            // same 32 records of a tile, with 8 halves of them.  A block's
+            // results keep to the one its size had.
+            if (kmode == kKernMixedP && (H == fill.warps) != (fill.H == fill.warps)) continue;
+            ForceConfig c = fill;
+            c.r = r;
+            c.H = H;
+            const int itile = c.warps / H * c.il * r;
+            const int n_itiles = (ni + itile - 1) / itile;
+            int last = 0;
+            for (int k = 1; k <= 12; ++k) {  // splits that give the busiest SM k CTAs
+                const int want = std::min(std::max(1, (int)((long long)num_sms * k / n_itiles)), ntiles);
+                const int per = (ntiles + want - 1) / want;
+                c.nsplit = (ntiles + per - 1) / per;
+                if (c.nsplit == last) continue;
+                last = c.nsplit;
+                const double t = shape_cost(q, kmode, c, ni, ntiles, num_sms);
+                if (t < least) {
+                    least = t;
+                    best = c;
+                }
+            }
+        }
+    return best;
 }
 
 // ---- batched (multi-item persistent) launches

@@ -155,6 +155,8 @@ int tile_size(int kmode);
 size_t jrec_bytes(int kmode);
 // Choose a launch configuration for ni x nj (heuristic; autotuner overrides).
 ForceConfig choose_config(int kmode, int ni, int nj_pad, int num_sms, bool nb);
+// The same with H and r from ni alone (j-split calls).
+ForceConfig fill_config(int kmode, int ni, int nj_pad, int num_sms);
 // Launch force (+ split reduction).  Returns a cudaError_t.  pot: the
 // potential only (acc, jerk written as zero, nn as 0); paired mixed or FP64
 // layout, cfg.r == 1, no neighbour lists.
