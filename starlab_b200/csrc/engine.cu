@@ -122,12 +122,8 @@ int Engine::open(int device, int nmax_hint) {
     G6_CHECK(cudaEventCreateWithFlags(&ev_ext_, cudaEventDisableTiming), "event");
     G6_CHECK(prepare_small_force(), "small call kernels");
     stage_cap_ = 16384;
-    G6_CHECK(cudaMallocHost(&h_stage_vals_, sizeof(double) * JF_COUNT * stage_cap_), "pinned stage");
-    G6_CHECK(cudaMallocHost(&h_stage_addr_, sizeof(int) * stage_cap_), "pinned stage");
-    G6_CHECK(cudaMallocHost(&h_stage_index_, sizeof(int) * stage_cap_), "pinned stage");
-    G6_CHECK(cudaMalloc(&d_stage_vals_, sizeof(double) * JF_COUNT * stage_cap_), "stage");
-    G6_CHECK(cudaMalloc(&d_stage_addr_, sizeof(int) * stage_cap_), "stage");
-    G6_CHECK(cudaMalloc(&d_stage_index_, sizeof(int) * stage_cap_), "stage");
+    G6_CHECK(cudaMallocHost(&h_stage_, sizeof(StagedJ) * stage_cap_), "pinned stage");
+    G6_CHECK(cudaMalloc(&d_stage_, sizeof(StagedJ) * stage_cap_), "stage");
     G6_CHECK(cudaMalloc(&d_energy_, sizeof(double) * (2 * kEnergyBlocks + 2)), "energy");
     G6_CHECK(cudaMallocHost(&h_energy_, sizeof(double) * 2), "energy");
     G6_CHECK(cudaMallocHost(&h_ref_count_, sizeof(int)), "refine");
@@ -156,10 +152,10 @@ void Engine::close() {
     auto dfree = [](void *p) { if (p) cudaFree(p); };
     auto hfree = [](void *p) { if (p) cudaFreeHost(p); };
     dfree(d_jraw_); dfree(d_jindex_); dfree(d_jrec_);
-    dfree(d_stage_vals_); dfree(d_stage_addr_); dfree(d_stage_index_);
+    dfree(d_stage_);
     dfree(d_irec_); dfree(d_out_); dfree(d_part_); dfree(d_tile_cnt_);
     dfree(d_nb_count_); dfree(d_nb_list_); dfree(d_nb_sorted_); dfree(d_nb_off_); dfree(d_bulk_);
-    hfree(h_stage_vals_); hfree(h_stage_addr_); hfree(h_stage_index_);
+    hfree(h_stage_);
     hfree(h_irec_); hfree(h_out_); hfree(h_nb_off_); hfree(h_nb_count_); hfree(h_bulk_);
     hfree(h_ieps2_); dfree(d_ieps2_); hfree(h_energy_); dfree(d_energy_);
     hfree(h_ref_count_); dfree(d_v2_); dfree(d_ref_small_); dfree(d_ref_items_); dfree(d_q_);
@@ -175,12 +171,13 @@ void Engine::close() {
     ev_ext_ = nullptr;
     cudaStreamDestroy(stream_);
     d_jraw_ = nullptr; d_jindex_ = nullptr; d_jrec_ = nullptr;
-    d_stage_vals_ = nullptr; d_stage_addr_ = nullptr; d_stage_index_ = nullptr;
+    d_stage_ = nullptr;
     d_irec_ = nullptr; d_out_ = nullptr; d_part_ = nullptr; d_tile_cnt_ = nullptr;
     d_nb_count_ = nullptr; d_nb_list_ = nullptr; d_nb_sorted_ = nullptr; d_nb_off_ = nullptr;
     d_bulk_ = nullptr; bulk_cap_ = 0; bulk_mark_.clear();
     h_bulk_ = nullptr; h_bulk_cap_ = 0; bulk_busy_ = false;
-    h_stage_vals_ = nullptr; h_stage_addr_ = nullptr; h_stage_index_ = nullptr;
+    h_stage_ = nullptr;
+    stage_busy_ = stage_until_done_ = false;
     h_irec_ = nullptr; h_out_ = nullptr; h_nb_off_ = nullptr; h_nb_count_ = nullptr;
     h_ieps2_ = nullptr; d_ieps2_ = nullptr; h_energy_ = nullptr; d_energy_ = nullptr;
     ev_stage_ = ev_begin_ = ev_pred0_ = ev_pred1_ = ev_force0_ = ev_force1_ = ev_done_ = nullptr;
@@ -205,7 +202,7 @@ int Engine::reset() {
         cudaStreamSynchronize(stream_);
     }
     small_parity_ = 0;
-    for (int k = 0; k < n_staged_; ++k) slot_of_[h_stage_addr_[k]] = -1;
+    for (int k = 0; k < n_staged_; ++k) slot_of_[h_stage_[k].addr] = -1;
     n_staged_ = 0;
     pending_ = false;
     pred_valid_ = pred64_valid_ = false;
@@ -270,7 +267,7 @@ int Engine::set_j(int address, int index, double tj, double mass, const double *
     if (!open_ && open(env_int("G6B200_DEVICE", 0), 0)) return -1;
     if (ensure_capacity(address)) return -1;
     if (stage_busy_) {
-        G6_CHECK(cudaEventSynchronize(ev_stage_), "stage wait");
+        G6_CHECK(cudaEventSynchronize(stage_until_done_ ? ev_done_ : ev_stage_), "stage wait");
         stage_busy_ = false;
     }
     int slot = slot_of_[address];
@@ -282,10 +279,10 @@ int Engine::set_j(int address, int index, double tj, double mass, const double *
         }
         slot = n_staged_++;
         slot_of_[address] = slot;
-        h_stage_addr_[slot] = address;
+        h_stage_[slot].addr = address;
     }
-    h_stage_index_[slot] = index;
-    double *r = h_stage_vals_ + (size_t)slot * JF_COUNT;
+    h_stage_[slot].index = index;
+    double *r = h_stage_[slot].vals;
     r[JF_T] = tj;
     r[JF_M] = mass;
     for (int c = 0; c < 3; ++c) {
@@ -306,22 +303,20 @@ int Engine::set_j(int address, int index, double tj, double mass, const double *
     return 0;
 }
 
-int Engine::flush_j() {
+int Engine::flush_j(bool in_call) {
     if (!open_ || n_staged_ == 0) return 0;
     G6_CHECK(cudaSetDevice(device_), "cudaSetDevice");
     const int n = n_staged_;
-    G6_CHECK(cudaMemcpyAsync(d_stage_vals_, h_stage_vals_, sizeof(double) * JF_COUNT * n,
-                             cudaMemcpyHostToDevice, stream_), "stage copy");
-    G6_CHECK(cudaMemcpyAsync(d_stage_addr_, h_stage_addr_, sizeof(int) * n, cudaMemcpyHostToDevice, stream_),
-             "stage copy");
-    G6_CHECK(cudaMemcpyAsync(d_stage_index_, h_stage_index_, sizeof(int) * n, cudaMemcpyHostToDevice, stream_),
-             "stage copy");
-    launch_scatter(stream_, n, d_stage_addr_, d_stage_index_, d_stage_vals_, d_jraw_, d_jindex_, cap_);
+    G6_CHECK(cudaMemcpyAsync(d_stage_, h_stage_, sizeof(StagedJ) * n, cudaMemcpyHostToDevice, stream_), "stage copy");
+    launch_scatter(stream_, n, d_stage_, d_jraw_, d_jindex_, cap_);
     G6_CHECK(cudaGetLastError(), "scatter launch");
-    G6_CHECK(cudaEventRecord(ev_stage_, stream_), "event");
+    // the staging records are free again when the copy is done: a call's own
+    // completion event says so too
     stage_busy_ = true;
-    stats_.h2d_bytes += (long long)n * (JF_COUNT * 8 + 8);
-    for (int k = 0; k < n; ++k) slot_of_[h_stage_addr_[k]] = -1;
+    stage_until_done_ = in_call;
+    if (!in_call) G6_CHECK(cudaEventRecord(ev_stage_, stream_), "event");
+    stats_.h2d_bytes += (long long)n * sizeof(StagedJ);
+    for (int k = 0; k < n; ++k) slot_of_[h_stage_[k].addr] = -1;
     n_staged_ = 0;
     pred_valid_ = pred64_valid_ = false;
     return 0;
@@ -627,13 +622,14 @@ int Engine::firsthalf_impl(int nj, int ni, const int *index, const double (*xi)[
     // staged updates' copies and scatter: without updates the copy path
     // (status clear, prediction, i-record copy) is as fast.
     call_small_ = small_enabled_ && n_staged_ > 0 && ni <= kSmallMax && n_staged_ <= kSmallMax;
-    if (!call_small_ && flush_j()) {
+    if (!call_small_ && flush_j(true)) {
         call_error_ = true;
         return -1;
     }
     int rc = launch_call();
     if (rc) {
         call_error_ = true;
+        cudaStreamSynchronize(stream_);  // ev_done_ may not have been recorded after the staging copy
         return rc;
     }
     pending_ = true;
@@ -695,13 +691,14 @@ int Engine::launch_call() {
     if (timed_) G6_CHECK(cudaEventRecord(ev_begin_, stream_), "event");
     const bool small = call_small_ && !call_sweep_;
     unsigned *status2 = reinterpret_cast<unsigned *>(d_out_ + L.status);
-    if (small) {
-        call_parity_ = small_parity_;
-        small_parity_ ^= 1;
-    } else {
+    // The call reports into one status word; its force (or small-call) kernel
+    // clears the other one for the next call.
+    call_parity_ = small_parity_;
+    small_parity_ ^= 1;
+    if (ni <= 0 && !small) {
         G6_CHECK(cudaMemsetAsync(d_out_, 0, 16, stream_), "memset");
         call_parity_ = 0;
-        small_parity_ = 1;  // word 1 stays clear: this call reports into word 0
+        small_parity_ = 1;
     }
     unsigned *status = status2 + call_parity_;
     pred_timed_ = false;
@@ -735,13 +732,13 @@ int Engine::launch_call() {
         sc.fs = fs;
         int order[kSmallMax];
         for (int k = 0; k < n_staged_; ++k) order[k] = k;
-        std::sort(order, order + n_staged_, [&](int a, int b) { return h_stage_addr_[a] < h_stage_addr_[b]; });
+        std::sort(order, order + n_staged_, [&](int a, int b) { return h_stage_[a].addr < h_stage_[b].addr; });
         for (int k = 0; k < n_staged_; ++k) {
             const int sl = order[k];
-            sc.addr[k] = h_stage_addr_[sl];
-            sc.index[k] = h_stage_index_[sl];
-            memcpy(sc.vals[k], h_stage_vals_ + (size_t)sl * JF_COUNT, sizeof(double) * JF_COUNT);
-            slot_of_[h_stage_addr_[sl]] = -1;
+            sc.addr[k] = h_stage_[sl].addr;
+            sc.index[k] = h_stage_[sl].index;
+            memcpy(sc.vals[k], h_stage_[sl].vals, sizeof(double) * JF_COUNT);
+            slot_of_[h_stage_[sl].addr] = -1;
         }
         memcpy(sc.irec, h_irec_, sizeof(IRec) * ni);
         if (call_g4_) memcpy(sc.ieps2, h_ieps2_, sizeof(double) * ni);
@@ -828,6 +825,7 @@ int Engine::launch_call() {
         p.nb_cap = nb_cap_;
         p.include_self = npipes_ > 48;
         p.status = status;
+        p.status_clear = small ? nullptr : status2 + (call_parity_ ^ 1);
         p.tile_counter = call_split_ ? nullptr : d_tile_cnt_;
         p.ieps2 = call_g4_ ? d_ieps2_ : nullptr;
         p.keep_partials = call_split_ ? 1 : 0;

@@ -61,6 +61,7 @@ template <int K, int IL, int R, bool NB, bool IDENT, int V>
 __global__ void __launch_bounds__(256, MinBlocks<K, R>::value) force_kernel(const ForceParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
     init_bars(smem);
+    if (p.status_clear && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *p.status_clear = 0u;
     int gt = 0;
     process_task<K, IL, R, NB, IDENT, V>(p, blockIdx.x, blockIdx.y, smem, gt);
 }

@@ -56,6 +56,7 @@ struct ForceParams {
     int nb_cap;
     int include_self;
     unsigned *status;
+    unsigned *status_clear;  // single calls: the other status word, cleared for the next call (or null)
     // Per-i-tile arrival counters (zero between calls).  When set and
     // nsplit > 1, the last CTA of an i-tile adds the split partials in split
     // order and writes the results, so no separate reduction launch is needed;
@@ -103,8 +104,12 @@ struct ForceConfig {
     int fine_ni = 0;    // batched plans: blocks of up to this many i take splits half as long
 };
 
-void launch_scatter(cudaStream_t s, int n, const int *addr, const int *index, const double *vals,
-                    double *jraw, int *jindex, int cap);
+// A staged j-update as it is copied to the device: one copy brings all.
+struct StagedJ {
+    double vals[JF_COUNT];  // JF_* fields
+    int addr, index;
+};
+void launch_scatter(cudaStream_t s, int n, const StagedJ *staged, double *jraw, int *jindex, int cap);
 // Device copies of a caller's j arrays for a bulk upload (addr/index/k18 may
 // be null: addresses 0..n-1, index = address, k18 = 0).
 struct BulkJ {

@@ -12,22 +12,19 @@
 
 namespace g6 {
 
-// Host staging records -> raw j-state.  One thread per (record, field):
-// reads are contiguous, writes land in 17 SoA rows.
-__global__ void scatter_j_kernel(int n, const int *__restrict__ addr,
-                                 const int *__restrict__ index,
-                                 const double *__restrict__ vals,
-                                 double *__restrict__ jraw, int *__restrict__ jindex,
-                                 int cap) {
-    long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    long long total = (long long)n * JF_COUNT;
-    if (t < total) {
-        int r = (int)(t / JF_COUNT);
-        int f = (int)(t - (long long)r * JF_COUNT);
-        int a = addr[r];
-        jraw[(size_t)f * cap + a] = vals[t];
-        if (f == 0) jindex[a] = index[r];
-    }
+// Host staging records -> raw j-state.  One thread per 8-byte word of a
+// record: reads are contiguous, writes land in 17 SoA rows.
+__global__ void scatter_j_kernel(int n, const StagedJ *__restrict__ staged, double *__restrict__ jraw,
+                                 int *__restrict__ jindex, int cap) {
+    constexpr int W = sizeof(StagedJ) / sizeof(double);
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (t >= (long long)n * W) return;
+    const int r = (int)(t / W), f = (int)(t - (long long)r * W);
+    const int a = staged[r].addr;
+    if (f < JF_COUNT)
+        jraw[(size_t)f * cap + a] = staged[r].vals[f];
+    else
+        jindex[a] = staged[r].index;
 }
 
 // Bulk upload: the caller's arrays, copied as they are (t[n], m[n], x, v,
@@ -231,13 +228,10 @@ void launch_irec_from_j(cudaStream_t s, const double *jraw, const int *jindex, i
     irec_from_j_kernel<<<(ni + 255) / 256, 256, 0, s>>>(jraw, jindex, cap, i0, ni, ti, out);
 }
 
-void launch_scatter(cudaStream_t s, int n, const int *addr, const int *index, const double *vals,
-                    double *jraw, int *jindex, int cap) {
+void launch_scatter(cudaStream_t s, int n, const StagedJ *staged, double *jraw, int *jindex, int cap) {
     if (n <= 0) return;
-    long long total = (long long)n * JF_COUNT;
-    int threads = 256;
-    unsigned blocks = (unsigned)((total + threads - 1) / threads);
-    scatter_j_kernel<<<blocks, threads, 0, s>>>(n, addr, index, vals, jraw, jindex, cap);
+    const long long total = (long long)n * (sizeof(StagedJ) / sizeof(double));
+    scatter_j_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(n, staged, jraw, jindex, cap);
 }
 
 void launch_scatter_bulk(cudaStream_t s, int n, const BulkJ &b, double *jraw, int *jindex, int cap) {
