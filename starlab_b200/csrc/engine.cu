@@ -816,10 +816,14 @@ int Engine::launch_call() {
         p.eps2 = call_eps2_;
         p.fs = fs;
         p.part = d_part_;
-        p.out_acc = reinterpret_cast<double *>(d_out_ + L.acc);
-        p.out_jerk = reinterpret_cast<double *>(d_out_ + L.jerk);
-        p.out_pot = reinterpret_cast<double *>(d_out_ + L.pot);
-        p.out_nn = reinterpret_cast<int *>(d_out_ + L.nn);
+        // A one-launch call's few results go straight to the pinned buffer
+        // (it has no copy waits and no fixed-point range, so no status to
+        // bring back); the others are copied there.
+        unsigned char *out = one_launch ? h_out_ : d_out_;
+        p.out_acc = reinterpret_cast<double *>(out + L.acc);
+        p.out_jerk = reinterpret_cast<double *>(out + L.jerk);
+        p.out_pot = reinterpret_cast<double *>(out + L.pot);
+        p.out_nn = reinterpret_cast<int *>(out + L.nn);
         p.nb_count = d_nb_count_;
         p.nb_list = d_nb_list_;
         p.nb_cap = nb_cap_;
@@ -911,7 +915,10 @@ int Engine::launch_call() {
         G6_CHECK(cudaEventRecord(ev_force1_, stream_), "event");
     }
     const size_t out_bytes = call_copy_ ? L.total : L.acc;  // status header only when not copying
-    G6_CHECK(cudaMemcpyAsync(h_out_, d_out_, out_bytes, cudaMemcpyDeviceToHost, stream_), "out copy");
+    if (one_launch)
+        memset(h_out_ + L.status, 0, L.acc - L.status);
+    else
+        G6_CHECK(cudaMemcpyAsync(h_out_, d_out_, out_bytes, cudaMemcpyDeviceToHost, stream_), "out copy");
     stats_.d2h_bytes += (long long)out_bytes;
     G6_CHECK(cudaEventRecord(ev_done_, stream_), "event");
     stats_.calls++;
