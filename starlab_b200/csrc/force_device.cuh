@@ -803,8 +803,10 @@ __device__ __forceinline__ void write_final(const ForceParams &p, int i, const P
 // a __threadfence in every thread before the count), 20.5 now; 1 x 65536 in
 // 64 splits 16.4 -> 12.3; 4096 x 65536 in 37, one segment, 0.636 -> 0.622 ms
 // (the 16-byte loads and the single release).
-// A function of its own, with the fields it needs passed by value: in line in
-// each lane shape's task it made the batched kernels spill.
+// In the batched and FP64 kernels a function of its own, with the fields it
+// needs passed by value: in line in each lane shape's task it made the
+// batched kernels spill.  In line in the single-call paired kernel, whose
+// pair loop a call costs 0.6 %.
 struct FoldArgs {
     const Partial *part;
     int ni, nj, nsplit;
@@ -813,7 +815,7 @@ struct FoldArgs {
     float *out_q;
     const int *out_map;
 };
-static __device__ __noinline__ void fold_splits(FoldArgs f, int ib, int itile, int slots, Partial *red) {
+__device__ __forceinline__ void fold_splits_inline(FoldArgs f, int ib, int itile, int slots, Partial *red) {
     ForceParams p{};  // what write_final reads
     p.nj = f.nj;
     p.out_acc = f.out_acc;
@@ -856,6 +858,10 @@ static __device__ __noinline__ void fold_splits(FoldArgs f, int ib, int itile, i
         if (mine && g < w) add_partial(red[g * it2 + k], red[(g + w) * it2 + k]);
     }
     if (mine && g == 0) write_final<true>(p, i, red[k]);
+}
+
+static __device__ __noinline__ void fold_splits(FoldArgs f, int ib, int itile, int slots, Partial *red) {
+    fold_splits_inline(f, ib, itile, slots, red);
 }
 
 // Resident CTAs per SM the register budget is sized for (3 for the paired
@@ -1129,9 +1135,13 @@ __device__ __forceinline__ bool process_task(const ForceParams &p, int itile_idx
         if (threadIdx.x == 0) s_last = arrive_count(&p.tile_counter[itile_idx]) == p.nsplit - 1;
         __syncthreads();
         if (s_last) {
-            fold_splits(FoldArgs{p.part, p.ni, p.nj, p.nsplit, p.out_acc, p.out_jerk, p.out_pot, p.out_nn, p.out_q,
-                                 K == kKernF64 ? p.out_map : nullptr},
-                        itile_idx * itile, itile, IL == 32 ? (int)blockDim.x : (int)blockDim.x / 2, red);
+            const FoldArgs f{p.part,     p.ni,      p.nj,     p.nsplit, p.out_acc, p.out_jerk,
+                             p.out_pot,  p.out_nn,  p.out_q,  K == kKernF64 ? p.out_map : nullptr};
+            const int slots = IL == 32 ? (int)blockDim.x : (int)blockDim.x / 2;
+            if constexpr ((V & kVarStats) != 0)
+                fold_splits_inline(f, itile_idx * itile, itile, slots, red);
+            else
+                fold_splits(f, itile_idx * itile, itile, slots, red);
             if (threadIdx.x == 0) p.tile_counter[itile_idx] = 0;
         }
     }
