@@ -936,13 +936,7 @@ int Engine::lasthalf(int ni, double (*acc)[3], double (*jerk)[3], double *pot, i
     int rc = wait_call();
     if (rc) return rc;
     const int n = std::min(ni, call_ni_);
-    OutLayout L(call_ni_);
-    parallel_ranges((size_t)n, 65536, [&](size_t lo, size_t hi, size_t) {
-        if (acc) memcpy(acc[lo], h_out_ + L.acc + 24 * lo, 24 * (hi - lo));
-        if (jerk) memcpy(jerk[lo], h_out_ + L.jerk + 24 * lo, 24 * (hi - lo));
-        if (pot) memcpy(pot + lo, h_out_ + L.pot + 8 * lo, 8 * (hi - lo));
-        if (nn) memcpy(nn + lo, h_out_ + L.nn + 4 * lo, 4 * (hi - lo));
-    });
+    copy_results(n, acc, jerk, pot, nn);
     ++lasthalf_count_;
     if (fault_lasthalf_at_ >= 0 && lasthalf_count_ == fault_lasthalf_at_) {
         last_error = "g6b200: injected lasthalf failure (G6B200_FAULT_LASTHALF)";
@@ -950,6 +944,19 @@ int Engine::lasthalf(int ni, double (*acc)[3], double (*jerk)[3], double *pot, i
     }
     if (fault_pot_at_ >= 0 && lasthalf_count_ == fault_pot_at_ && pot && n > 0) pot[0] = 1.0;
     return 0;
+}
+
+// The first n results of the call from the pinned buffer to the caller's
+// arrays, on a few host threads for large calls (the arrays are often fresh
+// memory, whose pages are touched here first).
+void Engine::copy_results(int n, double (*acc)[3], double (*jerk)[3], double *pot, int *nn) {
+    OutLayout L(call_ni_);
+    parallel_ranges((size_t)n, 32768, [&](size_t lo, size_t hi, size_t) {
+        if (acc) memcpy(acc[lo], h_out_ + L.acc + 24 * lo, 24 * (hi - lo));
+        if (jerk) memcpy(jerk[lo], h_out_ + L.jerk + 24 * lo, 24 * (hi - lo));
+        if (pot) memcpy(pot + lo, h_out_ + L.pot + 8 * lo, 8 * (hi - lo));
+        if (nn) memcpy(nn + lo, h_out_ + L.nn + 4 * lo, 4 * (hi - lo));
+    });
 }
 
 int Engine::wait_call() {
@@ -1027,13 +1034,7 @@ int Engine::sweep(int nj, int i0, int ni, double eps2, bool copy_out, double (*a
     if (launch_call()) return -1;
     int rc = wait_call();
     if (rc) return rc;
-    if (copy_out) {
-        OutLayout L(ni);
-        if (acc) memcpy(acc, h_out_ + L.acc, 24 * (size_t)ni);
-        if (jerk) memcpy(jerk, h_out_ + L.jerk, 24 * (size_t)ni);
-        if (pot) memcpy(pot, h_out_ + L.pot, 8 * (size_t)ni);
-        if (nn) memcpy(nn, h_out_ + L.nn, 4 * (size_t)ni);
-    }
+    if (copy_out) copy_results(ni, acc, jerk, pot, nn);
     return 0;
 }
 
@@ -1083,7 +1084,7 @@ int Engine::energies(int nj, double eps2, double *epot, double *ekin, double *po
     if (rc) return rc;
     if (epot) *epot = nj > 0 ? h_energy_[0] : 0.0;
     if (ekin) *ekin = nj > 0 ? h_energy_[1] : 0.0;
-    if (pot) memcpy(pot, h_out_ + OutLayout(nj).pot, 8 * (size_t)nj);
+    if (pot) copy_results(nj, nullptr, nullptr, pot, nullptr);
     return 0;
 }
 

@@ -147,6 +147,7 @@ class Engine {
     int ensure_nb_buffers();
     int launch_call();  // predictor (if stale) + force + nb compaction + D2H
     int wait_call();    // wait; handle the fixed-point range retry
+    void copy_results(int n, double (*acc)[3], double (*jerk)[3], double *pot, int *nn);
     int fail(const char *what, cudaError_t e);
     FixedScale scale() const;
     int choose_E(double xmax) const;

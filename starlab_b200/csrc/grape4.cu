@@ -32,15 +32,16 @@ namespace {
 constexpr int kBuffers = 64;
 constexpr int kJpMax = 1 << 20;
 
-struct JEntry {
-    int addr;
-    double x[3], v[3], a2[3], j6[3], m, t;
+// One DMA buffer, as the engine's bulk upload takes it.
+struct JBuffer {
+    std::vector<int> addr;
+    std::vector<double> x, v, a2, j6, m, t;  // vectors [n][3]
 };
 
 struct State {
     g6::Engine *eng = nullptr;
     double ti = 0;
-    std::vector<JEntry> buf[kBuffers];
+    JBuffer buf[kBuffers];
     int buff_used = 0;
     // last call: slots -> distinct records
     int ni = 0, nu = 0;
@@ -94,11 +95,13 @@ void check_buffer(int b, const char *who) {
 
 void commit(int b) {
     g6::Engine &e = engine();
-    for (const JEntry &q : g.buf[b]) {
-        if (e.set_j(q.addr, q.addr, q.t, q.m, nullptr, q.j6, q.a2, q.v, q.x))
-            die("(h3mjpdma_start) " + e.last_error);
-        g.j_updates++;
-    }
+    const JBuffer &q = g.buf[b];
+    const int n = (int)q.addr.size();
+    // as n set_j calls in order; large buffers go up in one piece
+    if (e.set_j_bulk(n, q.addr.data(), q.addr.data(), q.t.data(), q.m.data(), nullptr, q.j6.data(), q.a2.data(),
+                     q.v.data(), q.x.data()))
+        die("(h3mjpdma_start) " + e.last_error);
+    g.j_updates += n;
 }
 
 // Collect the results of the pending call into the per-record arrays.
@@ -145,7 +148,7 @@ void h3open_(void) { engine(); }
 
 void h3close_(void) {
     if (g.eng) g.eng->close();
-    for (auto &b : g.buf) b.clear();
+    for (auto &b : g.buf) b = JBuffer();
     g.buff_used = 0;
     g.pending = g.have_results = g.nb_read = false;
     g.ni = g.nu = 0;
@@ -177,21 +180,22 @@ void h3mjpdma_indirect_(int *nj, int *hostindex, double xj[][3], double vj[][3],
     }
     const int b = (buff_id && *buff_id >= 0) ? *buff_id : g.buff_used++;
     check_buffer(b, "h3mjpdma_indirect");
-    std::vector<JEntry> &B = g.buf[b];
-    B.resize(n);
+    for (int i = 0; i < n; ++i)
+        if (hostindex[i] < 1) die("(h3mjpdma_indirect) host index below 1");
+    JBuffer &B = g.buf[b];
+    B.addr.resize(n);
+    for (std::vector<double> *w : {&B.x, &B.v, &B.a2, &B.j6}) w->resize(3 * (size_t)n);
+    B.m.resize(n);
+    B.t.resize(n);
     for (int i = 0; i < n; ++i) {
         const int h = hostindex[i] - 1;
-        if (h < 0) die("(h3mjpdma_indirect) host index below 1");
-        JEntry &q = B[i];
-        q.addr = h;
-        for (int c = 0; c < 3; ++c) {
-            q.x[c] = xj[h][c];
-            q.v[c] = vj[h][c];
-            q.a2[c] = aj[h][c];
-            q.j6[c] = jj[h][c];
-        }
-        q.m = mj[h];
-        q.t = tj[h];
+        B.addr[i] = h;
+        memcpy(&B.x[3 * (size_t)i], xj[h], sizeof(double) * 3);
+        memcpy(&B.v[3 * (size_t)i], vj[h], sizeof(double) * 3);
+        memcpy(&B.a2[3 * (size_t)i], aj[h], sizeof(double) * 3);
+        memcpy(&B.j6[3 * (size_t)i], jj[h], sizeof(double) * 3);
+        B.m[i] = mj[h];
+        B.t[i] = tj[h];
     }
 }
 
@@ -226,21 +230,22 @@ void h3calc_firsthalf_(int *nj, int *ni, double xi[][3], double vi[][3], double 
     g6::Engine &e = engine();
     finish();  // a call whose results were never read
     g.slot.resize(n);
-    g.xu.clear();
-    g.vu.clear();
-    g.eu.clear();
-    g.hu.clear();
+    g.xu.resize(3 * (size_t)n);
+    g.vu.resize(3 * (size_t)n);
+    g.eu.resize(n);
+    g.hu.resize(n);
     int nu = 0;
     for (int k = 0; k < n; ++k) {
         if (k > 0 && same_slot(xi, vi, eps2, h2, k, k - 1)) {
             g.slot[k] = g.slot[k - 1];
             continue;
         }
-        g.slot[k] = nu++;
-        g.xu.insert(g.xu.end(), xi[k], xi[k] + 3);
-        g.vu.insert(g.vu.end(), vi[k], vi[k] + 3);
-        g.eu.push_back(2.0 * eps2[k]);
-        g.hu.push_back(2.0 * h2[k]);
+        g.slot[k] = nu;
+        memcpy(&g.xu[3 * (size_t)nu], xi[k], sizeof(double) * 3);
+        memcpy(&g.vu[3 * (size_t)nu], vi[k], sizeof(double) * 3);
+        g.eu[nu] = 2.0 * eps2[k];
+        g.hu[nu] = 2.0 * h2[k];
+        ++nu;
     }
     e.set_ti(g.ti);
     if (e.firsthalf_g4(m, nu, reinterpret_cast<const double(*)[3]>(g.xu.data()),

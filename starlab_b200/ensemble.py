@@ -10,7 +10,7 @@ import ctypes
 
 import numpy as np
 
-from .g6 import G6Error, load_library, _PREC
+from .g6 import G6Error, load_library, _PREC, _ptr as _p
 
 
 class EnsStats(ctypes.Structure):
@@ -34,9 +34,6 @@ def _bind(lib):
     lib.g6b200_ens_destroy.restype = None
     lib._ens_bound = True
 
-
-def _p(a):
-    return a.ctypes.data_as(ctypes.c_void_p)
 
 
 class Ensemble:

@@ -22,6 +22,8 @@ import os
 
 import numpy as np
 
+from .g6 import _full, _ptr as _p
+
 _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "lib", "libh3b200.so")
 
@@ -84,10 +86,6 @@ def _d(a, shape=None):
     return a
 
 
-def _p(a):
-    return a.ctypes.data_as(ctypes.c_void_p)
-
-
 def _ip(v):
     return ctypes.byref(ctypes.c_int(int(v)))
 
@@ -134,8 +132,7 @@ class H3Engine:
 
     def calc_firsthalf(self, nj, xi, vi, eps2, h2):
         ni = xi.shape[0]
-        self._hold = (_d(xi, (ni, 3)), _d(vi, (ni, 3)), _d(np.broadcast_to(np.asarray(eps2, float), (ni,))),
-                      _d(np.broadcast_to(np.asarray(h2, float), (ni,))))
+        self._hold = (_d(xi, (ni, 3)), _d(vi, (ni, 3)), _full(eps2, ni), _full(h2, ni))
         self.lib.h3calc_firsthalf_(_ip(nj), _ip(ni), *[_p(a) for a in self._hold])
 
     def calc_lasthalf(self, ni):

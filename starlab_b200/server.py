@@ -10,7 +10,7 @@ import ctypes
 
 import numpy as np
 
-from .g6 import G6Error, load_library, _PREC
+from .g6 import G6Error, load_library, _PREC, _full, _ptr as _p
 
 
 class SrvStats(ctypes.Structure):
@@ -41,9 +41,6 @@ def _bind(lib):
     lib._srv_bound = True
 
 
-def _p(a):
-    return None if a is None else a.ctypes.data_as(ctypes.c_void_p)
-
 
 class Server:
     def __init__(self, precision="mixed", hbm_budget=16 << 30, max_batch=1024, device=0):
@@ -66,7 +63,7 @@ class Server:
     def set_j(self, c, tj, mass, j6, a2, v, x, address=None):
         mass = np.ascontiguousarray(mass, np.float64)
         n = mass.shape[0]
-        tj = np.ascontiguousarray(np.broadcast_to(np.asarray(tj, np.float64), (n,)))
+        tj = _full(tj, n)
         arrs = [np.ascontiguousarray(q, np.float64).reshape(n, 3) for q in (j6, a2, v, x)]
         addr = None if address is None else np.ascontiguousarray(address, np.int32)
         rc = self.lib.g6b200_srv_set_j(self.h, int(c), n, _p(addr), _p(tj), _p(mass), *[_p(q) for q in arrs])
@@ -179,7 +176,7 @@ class ResidentServer:
     def set_j(self, c, tj, mass, j6, a2, v, x, address=None):
         mass = np.ascontiguousarray(mass, np.float64)
         n = mass.shape[0]
-        tj = np.ascontiguousarray(np.broadcast_to(np.asarray(tj, np.float64), (n,)))
+        tj = _full(tj, n)
         arrs = [np.ascontiguousarray(q, np.float64).reshape(n, 3) for q in (j6, a2, v, x)]
         addr = None if address is None else np.ascontiguousarray(address, np.int32)
         rc = self.lib.g6b200_res_set_j(self.h, int(c), n, _p(addr), _p(tj), _p(mass), *[_p(q) for q in arrs])

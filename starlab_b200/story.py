@@ -26,7 +26,7 @@ import ctypes
 
 import numpy as np
 
-from .g6 import load_library
+from .g6 import load_library, _ptr as _p
 
 RAW = 1
 
@@ -63,9 +63,6 @@ def _bind(lib):
     lib._story_bound = True
     return lib
 
-
-def _p(a):
-    return a.ctypes.data_as(ctypes.c_void_p)
 
 
 class Snapshot:
