@@ -699,10 +699,17 @@ __device__ __forceinline__ void to_partial(const StateMixedP &s, Partial &q) {
     q.qj = __int_as_float(s.qj);          // max m / r^3
 }
 __device__ __forceinline__ void to_partial(const StateF64 &s, Partial &q) {
-    constexpr double c1 = 1.0 / kSqrt3, c3 = c1 / 3.0;
-    q.acc[0] = c3 * s.Ax; q.acc[1] = c3 * s.Ay; q.acc[2] = c3 * s.Az;
-    q.jerk[0] = c3 * s.Jx; q.jerk[1] = c3 * s.Jy; q.jerk[2] = c3 * s.Jz;
-    q.pot = c1 * s.Pt;
+    // sqrt(t) and t sqrt(t) for t = kThird as it is rounded, in two doubles
+    // each: rounded to one they shift every sum the same way, by as much as
+    // all its terms' roundings together.
+    const auto scaled = [](double v, double hi, double lo) { return fma(v, hi, v * lo); };
+    constexpr double h1 = 0.5773502691896257, l1 = 1.7425591686159977e-17;
+    constexpr double h3 = 0.19245008972987523, l3 = 4.377263065132053e-18;
+    for (int c = 0; c < 3; ++c) {
+        q.acc[c] = scaled(c == 0 ? s.Ax : c == 1 ? s.Ay : s.Az, h3, l3);
+        q.jerk[c] = scaled(c == 0 ? s.Jx : c == 1 ? s.Jy : s.Jz, h3, l3);
+    }
+    q.pot = scaled(s.Pt, h1, l1);
     q.nn_r2 = s.nr2;
     q.nn_j = s.nj;
     q.qa = q.qj = 0.f;
