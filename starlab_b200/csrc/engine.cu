@@ -4,7 +4,9 @@
 // until lasthalf):
 //   set_j            host staging, deduplicated per address (last write
 //                    wins), pinned memory
-//   firsthalf        staged j -> device (one copy + scatter kernel);
+//   firsthalf        staged j -> device (one copy + scatter kernel; with up
+//                    to 64 i and 64 updates both ride on a launch's
+//                    parameter, and an FP64 call is that one launch);
 //                    predictor, only when the block time, nj, the j-state or
 //                    the fixed-point range changed (kira calls firsthalf once
 //                    per npipes-chunk of a block at the same time);

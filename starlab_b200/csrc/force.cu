@@ -15,8 +15,8 @@
 //
 // Work decomposition (one launch):
 //   gridDim.x  i-tiles;  gridDim.y  j-splits (contiguous address ranges,
-//              whole tiles; their partial sums are reduced in split order by
-//              reduce_partials_kernel, so the result is deterministic);
+//              whole tiles; the last CTA of an i-tile adds their partial
+//              sums in a fixed order, so the result is deterministic);
 //   CTA        NW warps = G i-groups x H j-subranges;
 //   warp       IL i-lanes x JL = 32/IL j-lanes; each thread owns R i's
 //              (register blocking: each j read from shared memory feeds R

@@ -201,16 +201,25 @@ __device__ __forceinline__ void interact_mixed(S &s, const JMixed &J, int jg, fl
 constexpr double kSqrt3 = 1.7320508075688772935;
 constexpr double kThird = 1.0 / 3.0;
 
-// sqrt(3) / r from r^2 / 3 (finite, normal, positive): the approximation's
-// relative error e/2, e = 1 - x y^2 below 2^-18, goes to 5/16 e^3 by
-// Householder's third-order step for x^(-1/2) (A. S. Householder, "The
-// Numerical Treatment of a Single Nonlinear Equation", 1970), y (1 + e/2 +
-// 3/8 e^2): below FP64's rounding.
-__device__ __forceinline__ double inv_dist_s3(double x) {
+// sqrt(3) / r (r^2 finite, normal, positive) from x = r^2 / 3 and q = c x.
+// The approximation y is taken of x; the residual e = c - q y^2 is that of q.
+// With q = x, one instruction less, the result is off by what 1/3 is no
+// double, 2.8e-17: enough for the potential, whose sum is scaled back by it
+// (to_partial).  But every 3 (dr.dv) / r^2 then is 5.5e-17 too large, and the
+// jerk's error against long doubles above the one with rsqrt() (1500 x 1500
+// over eight clusters, rms: 5.21e-16 against 4.80e-16); the forces take q =
+// r^2 itself: 4.64e-16, for 2 % of a 65536 x 65536 sweep.
+// y's low word is zero, so that y^2 is exact.  Its relative error e / 2c,
+// below 2^-19, goes to 5/16 (e/c)^3 by Householder's third-order step for
+// x^(-1/2) (A. S. Householder, "The Numerical Treatment of a Single
+// Nonlinear Equation", 1970), y (1 + (e/c)/2 + 3/8 (e/c)^2): below FP64's
+// rounding.
+template <int C>
+__device__ __forceinline__ double inv_dist_s3(double x, double q) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-(x * y), y, 1.0);
-    return fma(y * e, fma(e, 0.375, 0.5), y);
+    const double e = fma(-q, y * y, (double)C);
+    return fma(y * e, fma(e, 0.375 / (C * C), 0.5 / C), y);
 }
 
 __device__ __forceinline__ double r2_f64(double dx, double dy, double dz) {
@@ -273,11 +282,14 @@ __device__ __forceinline__ unsigned interact(StateF64 &s, const JRecF64 &J, int 
         r2 = out ? 1.0 : r2;
         hi = out ? 0xffffffffu : hi;
     }
-    const double y = inv_dist_s3(G4 ? r2 * kThird : __fma_rn(r2, kThird, s.eps2 * kThird));
     if constexpr (PO) {
+        const double x = __fma_rn(r2, kThird, s.eps2 * kThird);
+        const double y = inv_dist_s3<1>(x, x);
         s.Pt = __fma_rn(-m, y, s.Pt);
         return hi;
     }
+    if (!G4) r2 += s.eps2;
+    const double y = inv_dist_s3<3>(r2 * kThird, r2);
     const double dvx = J.vel.x - s.vx, dvy = J.vel.y - s.vy, dvz = J.vel.z - s.vz;
     const double rv = __fma_rn(dz, dvz, __fma_rn(dy, dvy, dx * dvx));
     const double q3 = y * y;  // 3 / r^2
@@ -681,6 +693,7 @@ __device__ __forceinline__ void take_min(double &r2, int &j, double o_r2, int o_
     }
 }
 
+template <bool PO>
 __device__ __forceinline__ void to_partial(const StateMixedBase &s, Partial &q) {
     q.acc[0] = s.Ax; q.acc[1] = s.Ay; q.acc[2] = s.Az;
     q.jerk[0] = s.Jx; q.jerk[1] = s.Jy; q.jerk[2] = s.Jz;
@@ -689,6 +702,7 @@ __device__ __forceinline__ void to_partial(const StateMixedBase &s, Partial &q) 
     q.nn_j = s.nj;
     q.qa = q.qj = 0.f;
 }
+template <bool PO>
 __device__ __forceinline__ void to_partial(const StateMixedP &s, Partial &q) {
     q.acc[0] = s.Ax; q.acc[1] = s.Ay; q.acc[2] = s.Az;
     q.jerk[0] = s.Jx; q.jerk[1] = s.Jy; q.jerk[2] = s.Jz;
@@ -698,13 +712,14 @@ __device__ __forceinline__ void to_partial(const StateMixedP &s, Partial &q) {
     q.qa = -2.f * __uint_as_float(s.qa);  // max m / r^2
     q.qj = __int_as_float(s.qj);          // max m / r^3
 }
+template <bool PO>
 __device__ __forceinline__ void to_partial(const StateF64 &s, Partial &q) {
-    // sqrt(t) and t sqrt(t) for t = kThird as it is rounded, in two doubles
-    // each: rounded to one they shift every sum the same way, by as much as
-    // all its terms' roundings together.
+    // 1/sqrt(3) and its cube (potential only: sqrt(kThird) as that is
+    // rounded), in two doubles each: rounded to one they shift every sum the
+    // same way, by as much as all its terms' roundings together.
     const auto scaled = [](double v, double hi, double lo) { return fma(v, hi, v * lo); };
-    constexpr double h1 = 0.5773502691896257, l1 = 1.7425591686159977e-17;
-    constexpr double h3 = 0.19245008972987523, l3 = 4.377263065132053e-18;
+    constexpr double h1 = 0.5773502691896257, l1 = PO ? 1.7425591686159977e-17 : 3.3450280739356345e-17;
+    constexpr double h3 = 0.19245008972987526, l3 = -7.353623497300496e-18;
     for (int c = 0; c < 3; ++c) {
         q.acc[c] = scaled(c == 0 ? s.Ax : c == 1 ? s.Ay : s.Az, h3, l3);
         q.jerk[c] = scaled(c == 0 ? s.Jx : c == 1 ? s.Jy : s.Jz, h3, l3);
@@ -1105,7 +1120,7 @@ __device__ __forceinline__ bool process_task(const ForceParams &p, int itile_idx
                 }
             }
         }
-        to_partial(st[r], q[r]);
+        to_partial<(V & kVarPot) != 0>(st[r], q[r]);
         if (JL > 1) warp_reduce<IL>(q[r]);
     }
     if (H > 1) {

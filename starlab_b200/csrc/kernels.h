@@ -322,9 +322,10 @@ __host__ __device__ inline int refine_tasks_wanted(int count, int nj_pad) {
     const long long wc = (long long)count * nj_pad / kMinTaskWork;
     return (int)(wc < kRefineMinTasks ? kRefineMinTasks : (wc > 592 ? 592 : wc));
 }
-// Split partial records the FP64 pass of a call of ni i can use: at most
-// 592 tasks over i-tiles of at most 64 i, so nsplit x flagged stays below
-// 592 x 64 + flagged.
+// Split partial records the FP64 pass of a call of ni i can use.  A pass of
+// few flagged i takes at most 592 tasks over i-tiles of at most 64 i, so that
+// its nsplit x flagged stays below 592 x 64 + flagged; one in whole waves is
+// cut no finer than these records hold (make_refine_item).
 __host__ __device__ inline size_t refine_partial_records(int ni) { return 64 * 600 + (size_t)ni; }
 
 // Neighbour lists: per-i sort + compaction into ascending address order.
