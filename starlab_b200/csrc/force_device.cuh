@@ -188,7 +188,7 @@ __device__ __forceinline__ void interact_mixed(S &s, const JMixed &J, int jg, fl
 // different register operands takes 3 cycles, one with two takes the FP64
 // pipe's 2 (measured: 3.04 and 2.04; an operand shared with the previous
 // instruction, or a literal one, is free).  The loop below is written
-// against that count -- about 70 cycles per j and warp:
+// against that count -- about 72 cycles per j and warp:
 //   * the inverse distance is the PTX approximation and one third-order step
 //     in line (11 cycles; rsqrt() measured 26, with a branch for the special
 //     values that keeps the pair terms of neighbouring j apart);
@@ -196,7 +196,7 @@ __device__ __forceinline__ void interact_mixed(S &s, const JMixed &J, int jg, fl
 //     its own;
 //   * the nearest neighbour is kept as the upper word of r^2 (one integer
 //     minimum per j instead of an FP64 compare and three selects).
-// 16384 x 262144: 10.56 -> 9.21 ms; potential only, 65536 x 65536: 5.39 ->
+// 16384 x 262144: 10.55 -> 9.40 ms; potential only, 65536 x 65536: 5.39 ->
 // 3.69 ms.
 constexpr double kSqrt3 = 1.7320508075688772935;
 constexpr double kThird = 1.0 / 3.0;
