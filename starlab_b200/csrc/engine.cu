@@ -707,6 +707,18 @@ int Engine::launch_call() {
     bool one_launch = false;
     const bool staged = small && n_staged_ > 0;
     bool need_pred;
+    // The staged updates are let go of, and the records taken as predicted,
+    // when the launch that does it has been accepted: a call that fails
+    // before keeps them for the next one.
+    auto small_launched = [&]() {
+        for (int k = 0; k < n_staged_; ++k) slot_of_[h_stage_[k].addr] = -1;
+        n_staged_ = 0;
+        stats_.h2d_bytes += (long long)sizeof(SmallCall);
+        if (need_pred) {
+            stats_.predictions++;
+            mark_predicted(nj, km);
+        }
+    };
     if (call_f64_) {
         need_pred = !pred64_valid_ || pred64_ti_ != ti_ || pred64_nj_ != nj || staged;
         if (staged) pred_valid_ = v2_valid_ = false;  // the updates land in the raw j-state: the mixed records are stale
@@ -740,12 +752,9 @@ int Engine::launch_call() {
             sc.addr[k] = h_stage_[sl].addr;
             sc.index[k] = h_stage_[sl].index;
             memcpy(sc.vals[k], h_stage_[sl].vals, sizeof(double) * JF_COUNT);
-            slot_of_[h_stage_[sl].addr] = -1;
         }
         memcpy(sc.irec, h_irec_, sizeof(IRec) * ni);
         if (call_g4_) memcpy(sc.ieps2, h_ieps2_, sizeof(double) * ni);
-        stats_.h2d_bytes += (long long)sizeof(SmallCall);
-        n_staged_ = 0;
         // FP64 force calls go further: updates, prediction and forces are one
         // launch (launch_small_force below) when each CTA's j-range fits its
         // shared memory.
@@ -760,10 +769,7 @@ int Engine::launch_call() {
             stats_.launches++;
             if (timed_) G6_CHECK(cudaEventRecord(ev_pred1_, stream_), "event");
             pred_timed_ = need_pred;
-        }
-        if (need_pred) {
-            stats_.predictions++;
-            mark_predicted(nj, km);
+            small_launched();
         }
     } else if (need_pred) {
         if (timed_) G6_CHECK(cudaEventRecord(ev_pred0_, stream_), "event");
@@ -838,10 +844,11 @@ int Engine::launch_call() {
         p.out_q = call_refine_ ? d_q_ : nullptr;
         if (call_nb_) G6_CHECK(cudaMemsetAsync(d_nb_count_, 0, sizeof(int) * ni, stream_), "memset");
         if (timed_) G6_CHECK(cudaEventRecord(ev_force0_, stream_), "event");
-        if (one_launch)
+        if (one_launch) {
             G6_CHECK(launch_small_force(stream_, cfg, p, small_call_, d_jraw_, d_jindex_, status2,
                                         n_nonident_ == 0 && !call_g4_, call_nb_), "force launch");
-        else
+            small_launched();
+        } else
             G6_CHECK(launch_force(stream_, km, cfg, p, n_nonident_ == 0 && !call_g4_, call_nb_, call_g4_, pot_k),
                      "force launch");
         if (timed_) G6_CHECK(cudaEventRecord(ev_force1_, stream_), "event");
