@@ -460,8 +460,11 @@ FixedScale Engine::scale() const {
 
 int Engine::ensure_call_buffers(int ni, bool nb, size_t part_bytes) {
     if (ni > call_cap_ || part_bytes > part_cap_ || (nb && nb_alloc_ < std::max(call_cap_, ni))) stats_.grows++;
+    // What is freed has no capacity until its successor is there: a failed
+    // allocation is the call's error, and the next call allocates again.
     if (ni > call_cap_) {
         int ncap = std::max(ni, npipes_);
+        call_cap_ = 0;
         if (h_irec_) cudaFreeHost(h_irec_);
         if (d_irec_) cudaFree(d_irec_);
         if (h_out_) cudaFreeHost(h_out_);
@@ -489,6 +492,7 @@ int Engine::ensure_call_buffers(int ni, bool nb, size_t part_bytes) {
     if (part_bytes > part_cap_) {
         if (d_part_) cudaFree(d_part_);
         d_part_ = nullptr;
+        part_cap_ = 0;
         size_t nb_ = part_bytes + part_bytes / 4;
         G6_CHECK(cudaMalloc(&d_part_, nb_), "partials");
         part_cap_ = nb_;
@@ -500,6 +504,9 @@ int Engine::ensure_call_buffers(int ni, bool nb, size_t part_bytes) {
         if (d_nb_off_) cudaFree(d_nb_off_);
         if (h_nb_off_) cudaFreeHost(h_nb_off_);
         if (h_nb_count_) cudaFreeHost(h_nb_count_);
+        d_nb_count_ = d_nb_list_ = d_nb_sorted_ = h_nb_count_ = nullptr;
+        d_nb_off_ = h_nb_off_ = nullptr;
+        nb_alloc_ = 0;
         const int n = call_cap_;
         G6_CHECK(cudaMalloc(&d_nb_count_, sizeof(int) * n), "nb");
         G6_CHECK(cudaMalloc(&d_nb_list_, sizeof(int) * (size_t)n * nb_cap_), "nb");
@@ -584,6 +591,7 @@ int Engine::firsthalf_impl(int nj, int ni, const int *index, const double (*xi)[
         if (hh > 0) nb = true;
     }
     if (ensure_call_buffers(ni, nb, 0)) {
+        call_nb_ = false;  // the last call's lists may be gone
         call_error_ = true;
         return -1;
     }

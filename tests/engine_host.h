@@ -110,6 +110,7 @@ void apply(const g6::SmallCall &sc, double *jraw, int *jindex) {
 // of, as its potential; no acc, jerk or neighbour.
 void force(const g6::ForceParams &p) {
     force_at = ++seq;
+    if (p.nsplit == 0 && nsplit > 1) memset(p.part, 0, (size_t)nsplit * p.ni * sizeof(g6::Partial));
     const g6::JRecF64 *r = static_cast<const g6::JRecF64 *>(p.jrec);
     for (int i = 0; i < p.ni; ++i) {
         double m = 0;
@@ -198,7 +199,10 @@ void launch_split_fix(cudaStream_t, int, int, int, long long, const Partial *, c
                       long long *) { abort(); }
 void launch_split_finish(cudaStream_t, int, int, long long, const long long *, const long long *, const long long *,
                          double *, double *, double *, int *) { abort(); }
-cudaError_t launch_nb_compact(cudaStream_t, int, const int *, const int *, int, long long *, int *) { abort(); }
+cudaError_t launch_nb_compact(cudaStream_t, int ni, const int *, const int *, int, long long *off, int *) {
+    memset(off, 0, sizeof(long long) * (ni + 1));
+    return cudaSuccess;
+}
 cudaError_t launch_nb_full_g4(cudaStream_t, const void *, int, const IRec &, double, int *, int, int *) { abort(); }
 void launch_copy_wait_selftest(cudaStream_t, unsigned *, unsigned long long) { abort(); }
 }  // namespace g6
