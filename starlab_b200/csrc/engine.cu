@@ -179,7 +179,7 @@ void Engine::close() {
     d_bulk_ = nullptr; bulk_cap_ = 0; bulk_mark_.clear();
     h_bulk_ = nullptr; h_bulk_cap_ = 0; bulk_busy_ = false;
     h_stage_ = nullptr;
-    stage_busy_ = stage_until_done_ = false;
+    stage_busy_ = false;
     h_irec_ = nullptr; h_out_ = nullptr; h_nb_off_ = nullptr; h_nb_count_ = nullptr;
     h_ieps2_ = nullptr; d_ieps2_ = nullptr; h_energy_ = nullptr; d_energy_ = nullptr;
     ev_stage_ = ev_begin_ = ev_pred0_ = ev_pred1_ = ev_force0_ = ev_force1_ = ev_done_ = nullptr;
@@ -269,7 +269,7 @@ int Engine::set_j(int address, int index, double tj, double mass, const double *
     if (!open_ && open(env_int("G6B200_DEVICE", 0), 0)) return -1;
     if (ensure_capacity(address)) return -1;
     if (stage_busy_) {
-        G6_CHECK(cudaEventSynchronize(stage_until_done_ ? ev_done_ : ev_stage_), "stage wait");
+        G6_CHECK(cudaEventSynchronize(ev_stage_), "stage wait");
         stage_busy_ = false;
     }
     int slot = slot_of_[address];
@@ -305,18 +305,18 @@ int Engine::set_j(int address, int index, double tj, double mass, const double *
     return 0;
 }
 
-int Engine::flush_j(bool in_call) {
+int Engine::flush_j() {
     if (!open_ || n_staged_ == 0) return 0;
     G6_CHECK(cudaSetDevice(device_), "cudaSetDevice");
     const int n = n_staged_;
     G6_CHECK(cudaMemcpyAsync(d_stage_, h_stage_, sizeof(StagedJ) * n, cudaMemcpyHostToDevice, stream_), "stage copy");
+    // The staging records are free again when the copy is done.  An event of
+    // its own says so: the call's completion event would keep a set_j beside
+    // a running call waiting for its forces.
+    G6_CHECK(cudaEventRecord(ev_stage_, stream_), "event");
+    stage_busy_ = true;
     launch_scatter(stream_, n, d_stage_, d_jraw_, d_jindex_, cap_);
     G6_CHECK(cudaGetLastError(), "scatter launch");
-    // the staging records are free again when the copy is done: a call's own
-    // completion event says so too
-    stage_busy_ = true;
-    stage_until_done_ = in_call;
-    if (!in_call) G6_CHECK(cudaEventRecord(ev_stage_, stream_), "event");
     stats_.h2d_bytes += (long long)n * sizeof(StagedJ);
     for (int k = 0; k < n; ++k) slot_of_[h_stage_[k].addr] = -1;
     n_staged_ = 0;
@@ -632,14 +632,13 @@ int Engine::firsthalf_impl(int nj, int ni, const int *index, const double (*xi)[
     // staged updates' copies and scatter: without updates the copy path
     // (status clear, prediction, i-record copy) is as fast.
     call_small_ = small_enabled_ && n_staged_ > 0 && ni <= kSmallMax && n_staged_ <= kSmallMax;
-    if (!call_small_ && flush_j(true)) {
+    if (!call_small_ && flush_j()) {
         call_error_ = true;
         return -1;
     }
     int rc = launch_call();
     if (rc) {
         call_error_ = true;
-        cudaStreamSynchronize(stream_);  // ev_done_ may not have been recorded after the staging copy
         return rc;
     }
     pending_ = true;

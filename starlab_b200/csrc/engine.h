@@ -48,9 +48,7 @@ class Engine {
 
     int set_j(int address, int index, double tj, double mass, const double *k18,
               const double *j6, const double *a2, const double *v, const double *x);
-    // in_call: a launch_call follows, whose completion event also marks the
-    // end of the staging copy.
-    int flush_j(bool in_call = false);
+    int flush_j();
     // Many j-particles at once (tj, mass [n]; k18, j6, a2, v, x [n][3] flat;
     // address/index/k18 may be null).  Same result as n set_j calls in
     // order: large uploads with distinct addresses go straight from the
@@ -194,8 +192,7 @@ class Engine {
     bool bulk_busy_ = false;           // ev_stage_ marks the end of its last copy
     std::vector<unsigned> bulk_mark_;  // duplicate-address check (generation stamps)
     unsigned bulk_gen_ = 0;
-    bool stage_busy_ = false;         // its last copy may be in flight: until ev_stage_, or
-    bool stage_until_done_ = false;   // (the copy went with a call) until ev_done_
+    bool stage_busy_ = false;         // its last copy may be in flight, until ev_stage_
 
     // per-call buffers
     int call_cap_ = 0;
