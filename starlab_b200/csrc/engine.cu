@@ -676,6 +676,20 @@ int Engine::ensure_jrec64() {
 }
 
 int Engine::launch_call() {
+    const int rc = launch_steps();
+    if (rc) {
+        // Part of the call may have been queued: let it finish, and leave
+        // both status words clear (this call's kernels may not have run) and
+        // no prediction taken for granted.
+        cudaStreamSynchronize(stream_);
+        if (d_out_) cudaMemsetAsync(d_out_, 0, 16, stream_);
+        small_parity_ = 0;
+        pred_valid_ = pred64_valid_ = v2_valid_ = false;
+    }
+    return rc;
+}
+
+int Engine::launch_steps() {
     const int ni = call_ni_, nj = call_nj_;
     call_refine_ = false;
     // Mixed mode: a call of fewer than mixed_min_work_ interactions runs in

@@ -143,7 +143,8 @@ class Engine {
     int firsthalf_impl(int nj, int ni, const int *index, const double (*xi)[3], const double (*vi)[3],
                        double eps2, const double *ieps2, const double *h2);
     int ensure_nb_buffers();
-    int launch_call();  // predictor (if stale) + force + nb compaction + D2H
+    int launch_call();   // launch_steps, undone as far as needed when a step fails
+    int launch_steps();  // predictor (if stale) + force + nb compaction + D2H
     int wait_call();    // wait; handle the fixed-point range retry
     void copy_results(int n, double (*acc)[3], double (*jerk)[3], double *pot, int *nn);
     int fail(const char *what, cudaError_t e);
