@@ -122,7 +122,6 @@ int Engine::open(int device, int nmax_hint) {
     cudaEvent_t *evs[] = {&ev_stage_, &ev_begin_, &ev_pred0_, &ev_pred1_, &ev_force0_, &ev_force1_, &ev_done_};
     for (cudaEvent_t *e : evs) G6_CHECK(cudaEventCreate(e), "event");
     G6_CHECK(cudaEventCreateWithFlags(&ev_ext_, cudaEventDisableTiming), "event");
-    G6_CHECK(prepare_small_force(), "small call kernels");
     stage_cap_ = 16384;
     G6_CHECK(cudaMallocHost(&h_stage_, sizeof(StagedJ) * stage_cap_), "pinned stage");
     G6_CHECK(cudaMalloc(&d_stage_, sizeof(StagedJ) * stage_cap_), "stage");
@@ -187,6 +186,7 @@ void Engine::close() {
     cap_ = 0; call_cap_ = 0; part_cap_ = 0; nb_alloc_ = 0;
     n_staged_ = 0; slot_of_.clear(); nonident_.clear(); n_nonident_ = 0;
     pred_valid_ = pred64_valid_ = false; pending_ = false; xmax_ = 0; E_ = -1000;
+    small_ready_ = 0;
     open_ = false;
 }
 
@@ -866,6 +866,11 @@ int Engine::launch_steps() {
         if (call_nb_) G6_CHECK(cudaMemsetAsync(d_nb_count_, 0, sizeof(int) * ni, stream_), "memset");
         if (timed_) G6_CHECK(cudaEventRecord(ev_force0_, stream_), "event");
         if (one_launch) {
+            const int variant = small_force_variant(cfg, n_nonident_ == 0 && !call_g4_, call_nb_, call_g4_);
+            if (!(small_ready_ >> variant & 1)) {
+                G6_CHECK(prepare_small_force(variant), "small call kernel");
+                small_ready_ |= 1u << variant;
+            }
             G6_CHECK(launch_small_force(stream_, cfg, p, small_call_, d_jraw_, d_jindex_, status2,
                                         n_nonident_ == 0 && !call_g4_, call_nb_), "force launch");
             small_launched();

@@ -273,6 +273,7 @@ class Engine {
 
     EngineStats stats_;
     SmallCall small_call_{};  // the parameter block of the last small call
+    unsigned small_ready_ = 0;  // one-launch variants prepared (bits)
 };
 
 }  // namespace g6

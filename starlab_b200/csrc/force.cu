@@ -458,14 +458,14 @@ bool small_force_fits(const ForceConfig &cfg, ForceParams p) {
     return cfg.r == 1 && cfg.H > 1 && p.nj_pad > 0 && small_smem_bytes(cfg, p, itile) <= kSmallSmemMax;
 }
 
-cudaError_t prepare_small_force() {
-    for (int il : {32, 8, 1})
-        for (int v = 0; v < 6; ++v) {
-            const cudaError_t e = cudaFuncSetAttribute(pick_small(il, v & 1, v & 2, v >= 4),
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmemMax);
-            if (e != cudaSuccess) return e;
-        }
-    return cudaSuccess;
+int small_force_variant(const ForceConfig &cfg, bool ident, bool nb, bool g4) {
+    return 6 * (cfg.il == 32 ? 0 : cfg.il == 8 ? 1 : 2) + (g4 ? 4 + nb : 2 * ident + nb);
+}
+
+cudaError_t prepare_small_force(int variant) {
+    const int il = variant / 6 == 0 ? 32 : variant / 6 == 1 ? 8 : 1, v = variant % 6;
+    return cudaFuncSetAttribute(pick_small(il, v & 1, v & 2, v >= 4), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                kSmallSmemMax);
 }
 
 cudaError_t launch_small_force(cudaStream_t s, const ForceConfig &cfg, ForceParams p, const SmallCall &sc,

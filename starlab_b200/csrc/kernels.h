@@ -169,11 +169,13 @@ cudaError_t launch_force(cudaStream_t s, int kmode, const ForceConfig &cfg, Forc
                          bool ident, bool nb, bool g4 = false, bool pot = false);
 // A small FP64 call as one launch: updates, prediction and forces (no
 // irec, ieps2 or records read; the records are written).  Fits when a CTA's
-// j-range fits into shared memory.  prepare: once per device before the
-// first launch.
+// j-range fits into shared memory.  prepare: once per device before the first
+// launch of a variant (which loads that kernel; all of them at open() made
+// opening an engine that runs none dearer).
 constexpr int kSmallSmemMax = 200 * 1024;
 bool small_force_fits(const ForceConfig &cfg, ForceParams p);
-cudaError_t prepare_small_force();
+int small_force_variant(const ForceConfig &cfg, bool ident, bool nb, bool g4);  // 0..17
+cudaError_t prepare_small_force(int variant);
 cudaError_t launch_small_force(cudaStream_t s, const ForceConfig &cfg, ForceParams p, const SmallCall &sc,
                                double *jraw, int *jindex, unsigned *status2, bool ident, bool nb);
 size_t partial_bytes(const ForceConfig &cfg, int ni);

@@ -144,7 +144,8 @@ size_t partial_bytes_fixed(int jper, int nj_pad, int ni) {
     return (size_t)std::max(1, (nj_pad + jper - 1) / jper) * ni * sizeof(Partial);
 }
 bool small_force_fits(const ForceConfig &, ForceParams) { return fake::small_fits; }
-cudaError_t prepare_small_force() {
+int small_force_variant(const ForceConfig &cfg, bool ident, bool nb, bool g4) { return nb + 2 * ident + 4 * g4; }
+cudaError_t prepare_small_force(int) {
     ++fake::prepared;
     return cudaSuccess;
 }
