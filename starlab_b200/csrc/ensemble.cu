@@ -847,9 +847,8 @@ int Ensemble::iteration(int mode, bool fused) {
 int Ensemble::start() {
     if (push_host_state()) return -1;
     if (iteration(1)) return -1;
+    ECHK(cudaMemsetAsync(d_.interactions, 0, sizeof *d_.interactions, stream_), "memset");
     ECHK(cudaStreamSynchronize(stream_), "start");
-    unsigned long long z = 0;
-    ECHK(cudaMemcpy(d_.interactions, &z, sizeof z, cudaMemcpyHostToDevice), "copy");
     return 0;
 }
 
@@ -1132,13 +1131,20 @@ int Ensemble::run_per_cluster(double t_end, EnsembleStats *st) {
         st->iterations = iters;
         st->launches = launches1 - launches0;
     }
-    // write the state back so energies/get_cluster see the baseline's result
-    ECHK(cudaMemcpy(d_.x, sx_.data(), sizeof(double) * 3 * N, cudaMemcpyHostToDevice), "copy");
-    ECHK(cudaMemcpy(d_.v, sv_.data(), sizeof(double) * 3 * N, cudaMemcpyHostToDevice), "copy");
-    ECHK(cudaMemcpy(d_.a, sa_.data(), sizeof(double) * 3 * N, cudaMemcpyHostToDevice), "copy");
-    ECHK(cudaMemcpy(d_.jk, sj_.data(), sizeof(double) * 3 * N, cudaMemcpyHostToDevice), "copy");
-    ECHK(cudaMemcpy(d_.t, st_.data(), sizeof(double) * N, cudaMemcpyHostToDevice), "copy");
-    ECHK(cudaMemcpy(d_.dt, sdt_.data(), sizeof(double) * N, cudaMemcpyHostToDevice), "copy");
+    // write the state back so energies/get_cluster see the baseline's result:
+    // on stream_, which they run on (a copy from pageable memory on the default
+    // stream may still be under way when it returns, and stream_ does not wait
+    // for that stream)
+    const auto back = [&](double *dst, const std::vector<double> &src) {
+        return cudaMemcpyAsync(dst, src.data(), sizeof(double) * src.size(), cudaMemcpyHostToDevice, stream_);
+    };
+    ECHK(back(d_.x, sx_), "copy");
+    ECHK(back(d_.v, sv_), "copy");
+    ECHK(back(d_.a, sa_), "copy");
+    ECHK(back(d_.jk, sj_), "copy");
+    ECHK(back(d_.t, st_), "copy");
+    ECHK(back(d_.dt, sdt_), "copy");
+    ECHK(cudaStreamSynchronize(stream_), "copy");
     return 0;
 }
 
