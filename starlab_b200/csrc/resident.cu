@@ -150,7 +150,10 @@ __device__ __forceinline__ void nap() { __nanosleep(1000); }
 
 // Grid barrier over co-resident CTAs (cooperative launch), bounded: false
 // when the other CTAs did not all arrive within limit_ns.  gen is thread 0's
-// count of barriers passed.
+// count of barriers passed.  What the CTAs wrote before it is ordered before
+// both kinds of reads behind it: ordinary loads (the fence after the wait and
+// the CTA barrier) and thread 0's bulk copies (the proxy fence: the predicted
+// records are written by ordinary stores).
 __device__ bool grid_barrier(const ResDev &d, unsigned &gen, unsigned long long limit_ns) {
     __shared__ int s_ok;
     __syncthreads();
@@ -172,6 +175,8 @@ __device__ bool grid_barrier(const ResDev &d, unsigned &gen, unsigned long long 
                 nap();
             }
         }
+        __threadfence();
+        fence_proxy_async_global();
         gen = target;
         s_ok = ok;
     }
