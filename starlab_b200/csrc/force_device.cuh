@@ -68,8 +68,8 @@ struct StateF64 {
     double eps2;  // softening: the call's, or (GRAPE-4 variant) this i's
     double Ax, Ay, Az, Jx, Jy, Jz, Pt;  // acc, jerk x 3 sqrt(3), pot x sqrt(3): see inv_dist_s3
     unsigned nhi;  // smallest upper word of r^2 so far
-    int nk, nk2;   // first j of the run that first reached it and of a second one that did (-1: none)
-    bool ntie;     // a third run reached it
+    int nk;        // first j of the run that first reached it (-1: none)
+    int nties;     // further runs that reached it: their first j are in process_task's ties[]
     double nr2;
     int nj, idx, i;
 };
@@ -114,8 +114,8 @@ __device__ __forceinline__ void load_i(StateF64 &s, const IRec &q, const ForcePa
     s.eps2 = p.eps2;
     s.Ax = s.Ay = s.Az = s.Jx = s.Jy = s.Jz = s.Pt = 0.0;
     s.nhi = kHiInf;
-    s.nk = s.nk2 = -1;
-    s.ntie = false;
+    s.nk = -1;
+    s.nties = 0;
     s.nr2 = DBL_MAX;
     s.nj = -1;
 }
@@ -545,9 +545,18 @@ __device__ __forceinline__ void fold(StateMixedBase &s) {
 // NnRun records it is compared with its value before the run, so the run
 // that first reached the minimum is known.  At the end of the task that
 // run's records are looked through again (nn_of_run, nn_scan_run): the same
-// j as a compare and select in every pair term.  A run divides a thread's
+// j as a compare and select in every pair term.  The FP64 minimum is of the
+// upper words alone, so runs that tie with it are listed and looked through
+// too; past kTies of them (a particle so far out that all its r^2 agree in
+// 20 bits) the thread's whole share is.  With two runs listed a lattice, where
+// most particles have more, took 13.26 ms for 64000 x 64000 and 0.50 ms for
+// 2000 x 64000; with eight 9.89 and 0.38, as distances without ties do.  The
+// far particles: 2000 of them 0.52 ms, 64000 x 64000 with 4096 10.9 ms.
+// Looking a tied run through at once instead cost 2000 x 64000 1.7 % without
+// any ties.  A run divides a thread's
 // share of a tile (a multiple of 16 records at 32 i-lanes, 4 at 8 i-lanes,
 // any number at 1).
+constexpr int kTies = 8;
 template <int K, int JL, int R, int V> struct NnRun {
     static constexpr int value =
         JL == 1 ? (K == kKernF64 && (R == 2 || (V & (kVarG4 | kVarPot)) != 0) ? 16 : 8) : (JL == 4 ? 4 : 1);
@@ -570,7 +579,7 @@ __device__ __forceinline__ void nn_of_run(StateMixedP &s, const JPairMixed *jrec
 template <int K, int R, int JL, bool CHK, bool NB, bool IDENT, int V>
 __device__ __forceinline__ void consume_tile(typename StateOf<K>::type (&st)[R],
                                              const typename Traits<K>::JRec *S, int kbase,
-                                             int per, int tb, const ForceParams &p) {
+                                             int per, int tb, const ForceParams &p, int (&ties)[R][kTies]) {
     if constexpr (K == kKernMixedP) {
         constexpr bool PO = (V & kVarPot) != 0;
         constexpr bool ST = (V & kVarStats) != 0;
@@ -639,14 +648,14 @@ __device__ __forceinline__ void consume_tile(typename StateOf<K>::type (&st)[R],
             if constexpr (!G4 && !PO) {
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
+                    const int run = tb + kbase + m0 * JL;
                     if (lo[r] < st[r].nhi) {
                         st[r].nhi = lo[r];
-                        st[r].nk = tb + kbase + m0 * JL;
-                        st[r].nk2 = -1;
-                        st[r].ntie = false;
+                        st[r].nk = run;
+                        st[r].nties = 0;
                     } else if (lo[r] == st[r].nhi) {
-                        st[r].ntie = st[r].nk2 >= 0;
-                        st[r].nk2 = st[r].nk2 >= 0 ? st[r].nk2 : tb + kbase + m0 * JL;
+                        if (st[r].nties < kTies) ties[r][st[r].nties] = run;
+                        if (st[r].nties <= kTies) ++st[r].nties;
                     }
                 }
             }
@@ -993,6 +1002,7 @@ __device__ __forceinline__ bool process_task(const ForceParams &p, int itile_idx
     const int i0 = itile_idx * itile + islot;
 
     State st[R];
+    int ties[R][kTies];  // FP64: runs whose smallest upper word ties with the least (NnRun)
     bool range_ok = true;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -1022,9 +1032,9 @@ __device__ __forceinline__ bool process_task(const ForceParams &p, int itile_idx
             chk = __any_sync(0xffffffffu, mine);
         }
         if (chk)
-            consume_tile<K, R, JL, true, NB, IDENT, V>(st, S, kbase, per, tb, p);
+            consume_tile<K, R, JL, true, NB, IDENT, V>(st, S, kbase, per, tb, p, ties);
         else
-            consume_tile<K, R, JL, false, NB, IDENT, V>(st, S, kbase, per, tb, p);
+            consume_tile<K, R, JL, false, NB, IDENT, V>(st, S, kbase, per, tb, p, ties);
     };
     bool ok = true;
     int t = 0;
@@ -1108,15 +1118,17 @@ __device__ __forceinline__ bool process_task(const ForceParams &p, int itile_idx
                     }
             }
             if constexpr (kRunNn) {
-                if (st[r].ntie) {
+                if (st[r].nties > kTies) {
 #pragma unroll 1
                     for (int t2 = 0; t2 < ntiles; ++t2)
 #pragma unroll 1
                         for (int m = 0; m < per; m += RUN) nn_scan_run<JL, RUN, IDENT>(st[r], all, first + t2 * T + m * JL);
                 } else if (st[r].nk >= 0) {
 #pragma unroll 1
-                    for (int k = st[r].nk; k >= 0; k = k == st[r].nk ? st[r].nk2 : -1)
+                    for (int u = -1; u < st[r].nties; ++u) {
+                        const int k = u < 0 ? st[r].nk : ties[r][u];
                         nn_scan_run<JL, RUN, IDENT>(st[r], records_of(k), k);
+                    }
                 }
             }
         }
