@@ -198,7 +198,6 @@ __device__ __forceinline__ void interact_mixed(S &s, const JMixed &J, int jg, fl
 //     minimum per j instead of an FP64 compare and three selects).
 // 16384 x 262144: 10.55 -> 9.40 ms; potential only, 65536 x 65536: 5.39 ->
 // 3.69 ms.
-constexpr double kSqrt3 = 1.7320508075688772935;
 constexpr double kThird = 1.0 / 3.0;
 
 // sqrt(3) / r (r^2 finite, normal, positive) from x = r^2 / 3 and q = c x.
@@ -231,7 +230,8 @@ __device__ __forceinline__ bool is_self(const StateF64 &s, const double4 &vel, i
     return IDENT ? jg == s.idx : vel.w == (double)s.idx;
 }
 
-// One pair term for any r^2 (zero, subnormal and infinite ones too).
+// One pair term for any r^2 (zero, subnormal and infinite ones too) and of any
+// size: not scaled.
 template <bool CHK, bool IDENT, bool G4, bool PO>
 __device__ __forceinline__ void interact_any(StateF64 &s, const double4 &pos, const double4 &vel, int jg) {
     const double dx = pos.x - s.x, dy = pos.y - s.y, dz = pos.z - s.z;
@@ -243,12 +243,12 @@ __device__ __forceinline__ void interact_any(StateF64 &s, const double4 &pos, co
     }
     const double rinv = rsqrt(r2);
     const double mr = mj * rinv;
-    s.Pt -= kSqrt3 * mr;
+    s.Pt -= mr;
     if constexpr (!PO) {
         const double dvx = vel.x - s.vx, dvy = vel.y - s.vy, dvz = vel.z - s.vz;
         const double rv = dx * dvx + dy * dvy + dz * dvz;
         const double r2inv = rinv * rinv;
-        const double mr3 = (3.0 * kSqrt3) * (mr * r2inv);
+        const double mr3 = mr * r2inv;
         const double a3 = -3.0 * rv * r2inv;
         s.Ax += mr3 * dx;
         s.Ay += mr3 * dy;
@@ -703,7 +703,7 @@ __device__ __forceinline__ void take_min(double &r2, int &j, double o_r2, int o_
 }
 
 template <bool PO>
-__device__ __forceinline__ void to_partial(const StateMixedBase &s, Partial &q) {
+__device__ __forceinline__ void to_partial(const StateMixedBase &s, Partial &q, bool) {
     q.acc[0] = s.Ax; q.acc[1] = s.Ay; q.acc[2] = s.Az;
     q.jerk[0] = s.Jx; q.jerk[1] = s.Jy; q.jerk[2] = s.Jz;
     q.pot = s.Pt;
@@ -712,7 +712,7 @@ __device__ __forceinline__ void to_partial(const StateMixedBase &s, Partial &q) 
     q.qa = q.qj = 0.f;
 }
 template <bool PO>
-__device__ __forceinline__ void to_partial(const StateMixedP &s, Partial &q) {
+__device__ __forceinline__ void to_partial(const StateMixedP &s, Partial &q, bool) {
     q.acc[0] = s.Ax; q.acc[1] = s.Ay; q.acc[2] = s.Az;
     q.jerk[0] = s.Jx; q.jerk[1] = s.Jy; q.jerk[2] = s.Jz;
     q.pot = s.Pt;
@@ -722,11 +722,11 @@ __device__ __forceinline__ void to_partial(const StateMixedP &s, Partial &q) {
     q.qj = __int_as_float(s.qj);          // max m / r^3
 }
 template <bool PO>
-__device__ __forceinline__ void to_partial(const StateF64 &s, Partial &q) {
+__device__ __forceinline__ void to_partial(const StateF64 &s, Partial &q, bool unscaled) {
     // 1/sqrt(3) and its cube (potential only: sqrt(kThird) as that is
     // rounded), in two doubles each: rounded to one they shift every sum the
     // same way, by as much as all its terms' roundings together.
-    const auto scaled = [](double v, double hi, double lo) { return fma(v, hi, v * lo); };
+    const auto scaled = [unscaled](double v, double hi, double lo) { return unscaled ? v : fma(v, hi, v * lo); };
     constexpr double h1 = 0.5773502691896257, l1 = PO ? 1.7425591686159977e-17 : 3.3450280739356345e-17;
     constexpr double h3 = 0.19245008972987526, l3 = -7.353623497300496e-18;
     for (int c = 0; c < 3; ++c) {
@@ -1099,14 +1099,21 @@ __device__ __forceinline__ bool process_task(const ForceParams &p, int itile_idx
     Partial q[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
+        bool unscaled = false;
         if constexpr (K == kKernMixedP && kRunNn) {
             if (st[r].nk >= 0) nn_of_run<JL, RUN, IDENT>(st[r], all);
         }
         if constexpr (K == kKernF64) {
             const int first = jb + kbase;
             // A sum that is not finite: some r^2 overflowed, vanished, or is
-            // negative or NaN.  Summed again with the pair term for any r^2.
-            if (!(fabs(st[r].Pt) <= DBL_MAX)) {
+            // negative or NaN, or a sum is too large for the scale.  Summed
+            // again, unscaled, with the pair term for any r^2.
+            double zero = 0.0 * st[r].Pt;  // NaN when a sum is not finite
+            if constexpr ((V & kVarPot) == 0)
+                zero += 0.0 * st[r].Ax + 0.0 * st[r].Ay + 0.0 * st[r].Az + 0.0 * st[r].Jx + 0.0 * st[r].Jy +
+                        0.0 * st[r].Jz;
+            unscaled = !(zero == 0.0);
+            if (unscaled) {
                 st[r].Ax = st[r].Ay = st[r].Az = st[r].Jx = st[r].Jy = st[r].Jz = st[r].Pt = 0.0;
 #pragma unroll 1
                 for (int t2 = 0; t2 < ntiles; ++t2)
@@ -1132,7 +1139,7 @@ __device__ __forceinline__ bool process_task(const ForceParams &p, int itile_idx
                 }
             }
         }
-        to_partial<(V & kVarPot) != 0>(st[r], q[r]);
+        to_partial<(V & kVarPot) != 0>(st[r], q[r], unscaled);
         if (JL > 1) warp_reduce<IL>(q[r]);
     }
     if (H > 1) {
