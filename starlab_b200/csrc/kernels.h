@@ -327,8 +327,40 @@ __host__ __device__ inline int refine_tasks_wanted(int count, int nj_pad) {
 // Split partial records the FP64 pass of a call of ni i can use.  A pass of
 // few flagged i takes at most 592 tasks over i-tiles of at most 64 i, so that
 // its nsplit x flagged stays below 592 x 64 + flagged; one in whole waves is
-// cut no finer than these records hold (make_refine_item).
+// cut no finer than these records hold (refine_tasks).
 __host__ __device__ inline size_t refine_partial_records(int ni) { return 64 * 600 + (size_t)ni; }
+// The pass's shape: i-tiles of 32, since few flagged particles leave fewer
+// lanes idle in them than in tiles of 64.
+__host__ __device__ inline ForceConfig refine_config(ForceConfig batch) {
+    batch.H = batch.warps;
+    return batch;
+}
+// Tasks of the pass over `count` flagged i of a call of calls_ni: those
+// wanted, or from one wave of its `slots` CTAs up, whole waves.  The number
+// of tasks is i-tiles x splits: the waves are the fewest that this comes
+// within 6 % of, as far as the partials reach, so that the last wave is not a
+// few tasks (78 flagged of 4096 against 262144: 312 tasks on 296 CTAs took 142
+// us, 294 tasks 86; 4818 of 262144 in 604 tasks 3.55 ms, in 1963 3.27).
+__host__ __device__ inline int refine_tasks(const ForceConfig &cfg, int count, int calls_ni, int nj_pad, int slots) {
+    int tasks = refine_tasks_wanted(count, nj_pad);
+    if (count <= 0 || tasks < slots) return tasks;
+    const int itile = batch_item_itile(kKernF64, cfg, count);
+    const int n_itiles = (count + itile - 1) / itile, ntiles = nj_pad / tile_of(kKernF64);
+    int best = 0;
+    for (int w = 1; w <= 16; ++w) {
+        const int sp = slots * w / n_itiles;  // splits that fill w waves
+        if (sp < 1) continue;
+        const int per = (ntiles + sp - 1) / sp, got = (ntiles + per - 1) / per;
+        if ((size_t)got * count > refine_partial_records(calls_ni) || (w > 1 && per < cfg.min_tiles)) break;
+        const int fill = (int)(1000ll * n_itiles * got / ((long long)slots * w));
+        if (fill > best) {
+            best = fill;
+            tasks = n_itiles * got;
+        }
+        if (fill >= 940) break;
+    }
+    return tasks;
+}
 
 // Neighbour lists: per-i sort + compaction into ascending address order.
 // offsets[ni+1] (exclusive scan of min(count, cap)), out[total].

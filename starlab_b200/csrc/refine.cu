@@ -62,36 +62,12 @@ __global__ void __launch_bounds__(kThreads) v2_total_kernel(double *work, int nj
 }
 
 // One FP64 work item for the flagged particles, sized by their count
-// (tasks wanted: refine_tasks_wanted, in whole waves of the pass's `slots`
-// CTAs from one wave up).  The item writes its results straight into the
-// flagged particles' rows of the call's outputs (out_map = the flag list).
-// The number of tasks is i-tiles x splits: the waves are the fewest that
-// this comes within 6 % of, as far as the partials reach, so that the last
-// wave is not a few tasks (78 flagged of 4096 against 262144: 312 tasks on
-// 296 CTAs took 142 us, 294 tasks 86; 4818 of 262144 in 604 tasks 3.55 ms,
-// in 1963 3.27).
+// (refine_tasks).  The item writes its results straight into the flagged
+// particles' rows of the call's outputs (out_map = the flag list).
 __device__ void make_refine_item(ForceParams p, ForceConfig cfg, int count, int calls_ni, int slots,
                                  ForceParams *items, int *pre, int *counter) {
     p.ni = count;
-    cfg.nsplit = refine_tasks_wanted(p.ni, p.nj_pad);
-    const int itile = batch_item_itile(kKernF64, cfg, count);
-    const int n_itiles = (count + itile - 1) / itile;
-    if (count > 0 && cfg.nsplit >= slots) {
-        const int ntiles = p.nj_pad / tile_of(kKernF64);
-        int best = 0;
-        for (int w = 1; w <= 16; ++w) {
-            const int sp = slots * w / n_itiles;  // splits that fill w waves
-            if (sp < 1 || (n_itiles > slots * w)) continue;
-            const int per = (ntiles + sp - 1) / sp, got = (ntiles + per - 1) / per;
-            if ((size_t)got * count > refine_partial_records(calls_ni) || (w > 1 && per < cfg.min_tiles)) break;
-            const int fill = (int)(1000ll * n_itiles * got / ((long long)slots * w));
-            if (fill > best) {
-                best = fill;
-                cfg.nsplit = n_itiles * got;
-            }
-            if (fill >= 940) break;
-        }
-    }
+    cfg.nsplit = refine_tasks(cfg, count, calls_ni, p.nj_pad, slots);
     int nt = 0;
     batch_plan(kKernF64, cfg, p, nt);
     items[0] = p;
@@ -152,8 +128,7 @@ void launch_refine_v2(cudaStream_t s, const double *jraw, int cap, int nj, doubl
 cudaError_t launch_refine(cudaStream_t s, const RefineArgs &r, int num_sms) {
     const int ni = r.ni;
     if (ni <= 0) return cudaSuccess;
-    ForceConfig cfg = batch_config(kKernF64);
-    cfg.H = cfg.warps;  // i-tiles of 32: few flagged particles leave fewer lanes idle than in tiles of 64
+    const ForceConfig cfg = refine_config(batch_config(kKernF64));
     const int slots = batch_ctas(kKernF64, cfg, num_sms);
     ForceParams base{};
     base.jrec = r.jrec64;
