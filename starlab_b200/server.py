@@ -156,6 +156,8 @@ class ResidentServer:
     Server, served by one persistent kernel that polls a request ring in
     pinned host memory (no launch per call or per batch)."""
 
+    ring_calls = 1024  # calls in flight: submit refuses one whose slot an unfinished call holds
+
     def __init__(self, precision="mixed", hbm_budget=16 << 30, max_batch=1024, device=0):
         self.lib = load_library()
         _bind_res(self.lib)

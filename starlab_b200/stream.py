@@ -18,7 +18,6 @@ import numpy as np
 from . import ics
 
 EPS2 = 1e-6
-MAX_IN_FLIGHT = 960
 
 
 def make_clusters(k, seed, n_lo=512, n_hi=65536):
@@ -55,6 +54,11 @@ def _inputs(cl, ni, i0, ti):
 
 
 def run_served(server, clusters, calls):
+    """The stream through a server.  A call's latency is counted from its
+    arrival, as run_sequential's: its time in the server and the time by which
+    it was submitted late.  A server with a request ring takes that many calls
+    in flight; further ones wait here."""
+    ring = getattr(server, "ring_calls", None)
     ids = []
     for (m, x, v, a, j) in clusters:
         c = server.open_cluster(len(m), EPS2)
@@ -72,12 +76,13 @@ def run_served(server, clusters, calls):
                 break
             time.sleep(min(dt, 0.0005))
         idx, xs, vs = pre[q]
-        if q >= MAX_IN_FLIGHT:  # the resident server's request ring holds 1024 calls
-            futs[q - MAX_IN_FLIGHT][1].result()
+        if ring and q >= ring:
+            futs[q - ring][1].result()
+        lat[q] = time.perf_counter() - (t0 + ta)
         rid = server.submit(ids[c], ti, len(clusters[c][0]), idx, xs, vs)
         futs.append((q, pool.submit(server.wait, rid)))
     for q, f in futs:
-        lat[q] = f.result()[4]
+        lat[q] += f.result()[4]
     wall = time.perf_counter() - t0
     pool.shutdown()
     inter = sum(ni * len(clusters[c][0]) for (_, c, ni, _, _) in calls)
