@@ -123,7 +123,9 @@ int Engine::open(int device, int nmax_hint) {
     for (cudaEvent_t *e : evs) G6_CHECK(cudaEventCreate(e), "event");
     G6_CHECK(cudaEventCreateWithFlags(&ev_ext_, cudaEventDisableTiming), "event");
     stage_cap_ = 16384;
-    G6_CHECK(cudaMallocHost(&h_stage_, sizeof(StagedJ) * stage_cap_), "pinned stage");
+    G6_CHECK(cudaMallocHost(&h_stage_, sizeof(StagedJ) * (stage_cap_ + 1)), "pinned stage");
+    h_stage_copied_ = reinterpret_cast<unsigned *>(h_stage_ + stage_cap_);
+    *h_stage_copied_ = stage_seq_ = 0;
     G6_CHECK(cudaMalloc(&d_stage_, sizeof(StagedJ) * stage_cap_), "stage");
     G6_CHECK(cudaMalloc(&d_energy_, sizeof(double) * (2 * kEnergyBlocks + 2)), "energy");
     G6_CHECK(cudaMallocHost(&h_energy_, sizeof(double) * 2), "energy");
@@ -268,16 +270,11 @@ int Engine::set_j(int address, int index, double tj, double mass, const double *
     }
     if (!open_ && open(env_int("G6B200_DEVICE", 0), 0)) return -1;
     if (ensure_capacity(address)) return -1;
-    if (stage_busy_) {
-        G6_CHECK(cudaEventSynchronize(ev_stage_), "stage wait");
-        stage_busy_ = false;
-    }
+    if (stage_busy_ && stage_wait()) return -1;
     int slot = slot_of_[address];
     if (slot < 0) {
         if (n_staged_ == stage_cap_) {
-            if (flush_j()) return -1;
-            G6_CHECK(cudaEventSynchronize(ev_stage_), "stage wait");
-            stage_busy_ = false;
+            if (flush_j() || stage_wait()) return -1;
         }
         slot = n_staged_++;
         slot_of_[address] = slot;
@@ -305,17 +302,27 @@ int Engine::set_j(int address, int index, double tj, double mass, const double *
     return 0;
 }
 
+int Engine::stage_wait() {
+    // (a stream with nothing left to do, or an error, ends the wait too)
+    while (__atomic_load_n(h_stage_copied_, __ATOMIC_ACQUIRE) != stage_seq_) {
+        const cudaError_t e = cudaStreamQuery(stream_);
+        if (e == cudaSuccess) break;
+        if (e != cudaErrorNotReady) return fail("stage wait", e);
+    }
+    stage_busy_ = false;
+    return 0;
+}
+
 int Engine::flush_j() {
     if (!open_ || n_staged_ == 0) return 0;
     G6_CHECK(cudaSetDevice(device_), "cudaSetDevice");
     const int n = n_staged_;
     G6_CHECK(cudaMemcpyAsync(d_stage_, h_stage_, sizeof(StagedJ) * n, cudaMemcpyHostToDevice, stream_), "stage copy");
-    // The staging records are free again when the copy is done.  An event of
-    // its own says so: the call's completion event would keep a set_j beside
-    // a running call waiting for its forces.
-    G6_CHECK(cudaEventRecord(ev_stage_, stream_), "event");
+    // The staging records are free again when the copy is done, which the
+    // scatter kernel says: a call's completion event would keep a set_j beside
+    // the running call waiting for its forces.
     stage_busy_ = true;
-    launch_scatter(stream_, n, d_stage_, d_jraw_, d_jindex_, cap_);
+    launch_scatter(stream_, n, d_stage_, d_jraw_, d_jindex_, cap_, h_stage_copied_, ++stage_seq_);
     G6_CHECK(cudaGetLastError(), "scatter launch");
     stats_.h2d_bytes += (long long)n * sizeof(StagedJ);
     for (int k = 0; k < n; ++k) slot_of_[h_stage_[k].addr] = -1;

@@ -193,7 +193,10 @@ class Engine {
     bool bulk_busy_ = false;           // ev_stage_ marks the end of its last copy
     std::vector<unsigned> bulk_mark_;  // duplicate-address check (generation stamps)
     unsigned bulk_gen_ = 0;
-    bool stage_busy_ = false;         // its last copy may be in flight, until ev_stage_
+    bool stage_busy_ = false;          // its last copy may be in flight (stage_wait)
+    unsigned *h_stage_copied_ = nullptr;  // pinned: the last flush whose copy is done
+    unsigned stage_seq_ = 0;           // the last flush
+    int stage_wait();                  // until the staging records are free again
 
     // per-call buffers
     int call_cap_ = 0;

@@ -109,7 +109,10 @@ struct StagedJ {
     double vals[JF_COUNT];  // JF_* fields
     int addr, index;
 };
-void launch_scatter(cudaStream_t s, int n, const StagedJ *staged, double *jraw, int *jindex, int cap);
+// Staged updates to the raw j-state; writes seq to *copied (pinned host
+// memory) when it starts, that is when the copy queued before it is done.
+void launch_scatter(cudaStream_t s, int n, const StagedJ *staged, double *jraw, int *jindex, int cap,
+                    unsigned *copied, unsigned seq);
 // Device copies of a caller's j arrays for a bulk upload (addr/index/k18 may
 // be null: addresses 0..n-1, index = address, k18 = 0).
 struct BulkJ {

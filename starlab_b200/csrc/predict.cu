@@ -13,11 +13,15 @@
 namespace g6 {
 
 // Host staging records -> raw j-state.  One thread per 8-byte word of a
-// record: reads are contiguous, writes land in 17 SoA rows.
+// record: reads are contiguous, writes land in 17 SoA rows.  The kernel runs
+// behind the copy of the records, so its first thread's word in pinned memory
+// tells the host that the copy is done (an event recorded in between cost a
+// call of 200 i 3 us of 66).
 __global__ void scatter_j_kernel(int n, const StagedJ *__restrict__ staged, double *__restrict__ jraw,
-                                 int *__restrict__ jindex, int cap) {
+                                 int *__restrict__ jindex, int cap, volatile unsigned *copied, unsigned seq) {
     constexpr int W = sizeof(StagedJ) / sizeof(double);
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (t == 0) *copied = seq;
     if (t >= (long long)n * W) return;
     const int r = (int)(t / W), f = (int)(t - (long long)r * W);
     const int a = staged[r].addr;
@@ -228,10 +232,11 @@ void launch_irec_from_j(cudaStream_t s, const double *jraw, const int *jindex, i
     irec_from_j_kernel<<<(ni + 255) / 256, 256, 0, s>>>(jraw, jindex, cap, i0, ni, ti, out);
 }
 
-void launch_scatter(cudaStream_t s, int n, const StagedJ *staged, double *jraw, int *jindex, int cap) {
+void launch_scatter(cudaStream_t s, int n, const StagedJ *staged, double *jraw, int *jindex, int cap,
+                    unsigned *copied, unsigned seq) {
     if (n <= 0) return;
     const long long total = (long long)n * (sizeof(StagedJ) / sizeof(double));
-    scatter_j_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(n, staged, jraw, jindex, cap);
+    scatter_j_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(n, staged, jraw, jindex, cap, copied, seq);
 }
 
 void launch_scatter_bulk(cudaStream_t s, int n, const BulkJ &b, double *jraw, int *jindex, int cap) {

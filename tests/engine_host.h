@@ -37,6 +37,7 @@ cudaError_t fake_cudaDeviceGetAttribute(int *v, cudaDeviceAttr, int) { *v = 148;
 cudaError_t fake_cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { *s = reinterpret_cast<cudaStream_t>(1); return cudaSuccess; }
 cudaError_t fake_cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t fake_cudaStreamSynchronize(cudaStream_t) { fake::waited_for = fake::seq; return cudaSuccess; }
+cudaError_t fake_cudaStreamQuery(cudaStream_t) { fake::waited_for = fake::seq; return cudaSuccess; }
 cudaError_t fake_cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
 cudaError_t fake_cudaEventCreate(cudaEvent_t *e) { *e = reinterpret_cast<cudaEvent_t>(new fake::Event); return cudaSuccess; }
 cudaError_t fake_cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) { return fake_cudaEventCreate(e); }
@@ -93,6 +94,7 @@ cudaError_t fake_cudaMemcpy2DAsync(void *d, size_t dp, const void *s, size_t sp,
 #define cudaSetDevice fake_cudaSetDevice
 #define cudaStreamCreateWithFlags fake_cudaStreamCreateWithFlags
 #define cudaStreamDestroy fake_cudaStreamDestroy
+#define cudaStreamQuery fake_cudaStreamQuery
 #define cudaStreamSynchronize fake_cudaStreamSynchronize
 #define cudaStreamWaitEvent fake_cudaStreamWaitEvent
 #include "engine.cu"
@@ -180,8 +182,10 @@ void launch_predict(cudaStream_t, int, const double *jraw, const int *, int cap,
     ++fake::seq;
     fake::predict(jraw, cap, nj, nj_pad, jrec);
 }
-void launch_scatter(cudaStream_t, int n, const StagedJ *staged, double *jraw, int *jindex, int cap) {
+void launch_scatter(cudaStream_t, int n, const StagedJ *staged, double *jraw, int *jindex, int cap, unsigned *copied,
+                    unsigned seq) {
     ++fake::seq;
+    *copied = seq;
     ++fake::scatters;
     for (int k = 0; k < n; ++k) {
         for (int f = 0; f < JF_COUNT; ++f) jraw[(size_t)f * cap + staged[k].addr] = staged[k].vals[f];
