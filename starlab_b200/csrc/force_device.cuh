@@ -1043,9 +1043,12 @@ __device__ __forceinline__ bool process_task(const ForceParams &p, int itile_idx
         __syncthreads();
         for (; t < ntiles; ++t) consume(tiles + t * U, jb + t * T);
     } else {
-        // The previous task's epilogue may still read the tile area.
+        // The previous task's epilogue may still read the tile area, and has
+        // written its reductions there: ordinary stores, ordered before the
+        // copies by the proxy fence.
         __syncthreads();
         if (threadIdx.x == 0 && ntiles > 0) {
+            if (g0 > 0) fence_proxy_async();
             const int b = g0 & 1;
             mbar_arrive_expect_tx(&bars[b], kTileBytes);
             bulk_g2s(tiles + b * U, jrec + jb / JPU, kTileBytes, &bars[b]);
