@@ -549,11 +549,11 @@ __device__ __forceinline__ void fold(StateMixedBase &s) {
 // upper words alone, so runs that tie with it are listed and looked through
 // too; past kTies of them (a particle so far out that all its r^2 agree in
 // 20 bits) the thread's whole share is.  With two runs listed a lattice, where
-// most particles have more, took 13.26 ms for 64000 x 64000 and 0.50 ms for
-// 2000 x 64000; with eight 9.89 and 0.38, as distances without ties do.  The
-// far particles: 2000 of them 0.52 ms, 64000 x 64000 with 4096 10.9 ms.
-// Looking a tied run through at once instead cost 2000 x 64000 1.7 % without
-// any ties.  A run divides a thread's
+// most particles have more, took 13.26 ms for 64000 x 64000 and 0.49 ms for
+// 2000 x 64000; with eight 9.78 and 0.378 (distances without ties 9.74 and
+// 0.371).  The far particles: 2000 of them 0.51 ms, 64000 x 64000 with 4096
+// 10.6 ms.  Looking a tied run through at once instead cost 2000 x 64000 1.7 %
+// without any ties.  A run divides a thread's
 // share of a tile (a multiple of 16 records at 32 i-lanes, 4 at 8 i-lanes,
 // any number at 1).
 constexpr int kTies = 8;
@@ -649,13 +649,17 @@ __device__ __forceinline__ void consume_tile(typename StateOf<K>::type (&st)[R],
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
                     const int run = tb + kbase + m0 * JL;
-                    if (lo[r] < st[r].nhi) {
-                        st[r].nhi = lo[r];
-                        st[r].nk = run;
-                        st[r].nties = 0;
-                    } else if (lo[r] == st[r].nhi) {
-                        if (st[r].nties < kTies) ties[r][st[r].nties] = run;
-                        if (st[r].nties <= kTies) ++st[r].nties;
+                    // one branch, rarely taken: 2000 x 64000 0.371 ms, with selects
+                    // for the smaller word and a branch for the tie 0.378
+                    if (__builtin_expect(lo[r] <= st[r].nhi, 0)) {
+                        if (lo[r] < st[r].nhi) {
+                            st[r].nhi = lo[r];
+                            st[r].nk = run;
+                            st[r].nties = 0;
+                        } else {
+                            if (st[r].nties < kTies) ties[r][st[r].nties] = run;
+                            if (st[r].nties <= kTies) ++st[r].nties;
+                        }
                     }
                 }
             }

@@ -172,12 +172,14 @@ cudaError_t launch_force(cudaStream_t s, int kmode, const ForceConfig &cfg, Forc
                          bool ident, bool nb, bool g4 = false, bool pot = false);
 // A small FP64 call as one launch: updates, prediction and forces (no
 // irec, ieps2 or records read; the records are written).  Fits when a CTA's
-// j-range fits into shared memory.  prepare: once per device before the first
-// launch of a variant (which loads that kernel; all of them at open() made
-// opening an engine that runs none dearer).
+// j-range fits into shared memory: faster than updates and prediction, then
+// forces, at every size measured that fits (1 to 64 i, 1 to 64 updates, 256 to
+// 480000 j: 1.2 times at 480000 x 64, 1.8 at 1024 x 24).  prepare: once per
+// device before the first launch of a variant (variants 0..17); the first one
+// loads the force kernels, 22 ms, which all of them at open() moved there.
 constexpr int kSmallSmemMax = 200 * 1024;
 bool small_force_fits(const ForceConfig &cfg, ForceParams p);
-int small_force_variant(const ForceConfig &cfg, bool ident, bool nb, bool g4);  // 0..17
+int small_force_variant(const ForceConfig &cfg, bool ident, bool nb, bool g4);
 cudaError_t prepare_small_force(int variant);
 cudaError_t launch_small_force(cudaStream_t s, const ForceConfig &cfg, ForceParams p, const SmallCall &sc,
                                double *jraw, int *jindex, unsigned *status2, bool ident, bool nb);
