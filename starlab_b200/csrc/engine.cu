@@ -1017,6 +1017,9 @@ int Engine::wait_call() {
             stats_.range_retries++;
             E_ += 2;
             pred_valid_ = false;
+            // A small call's updates are in the raw j-state by now; those
+            // staged since are the next call's (and may be more than kSmallMax).
+            call_small_ = false;
             if (launch_call()) return 2;
             continue;
         }

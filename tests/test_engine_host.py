@@ -12,7 +12,7 @@ from starlab_b200 import build
 HERE = os.path.dirname(os.path.abspath(__file__))
 
 
-@pytest.mark.parametrize("program", ["failed_call", "no_memory", "upload_during_call", "status_words", "open"])
+@pytest.mark.parametrize("program", ["failed_call", "no_memory", "upload_during_call", "status_words", "open", "retry"])
 def test_engine_host(program, tmp_path):
     nvcc = build.NVCC if os.path.exists(build.NVCC) else shutil.which("nvcc")
     if not nvcc:
