@@ -1052,7 +1052,7 @@ __device__ __forceinline__ bool process_task(const ForceParams &p, int itile_idx
         // copies by the proxy fence.
         __syncthreads();
         if (threadIdx.x == 0 && ntiles > 0) {
-            if (g0 > 0) fence_proxy_async();
+            if (g0 != 0) fence_proxy_async();
             const int b = g0 & 1;
             mbar_arrive_expect_tx(&bars[b], kTileBytes);
             bulk_g2s(tiles + b * U, jrec + jb / JPU, kTileBytes, &bars[b]);
