@@ -252,9 +252,10 @@ ForceConfig fill_config(int kmode, int ni, int nj_pad, int num_sms) {
     c.r = ((kmode == kKernMixedDS || kmode == kKernF64) && c.il == 32 && ni >= 8192) ? 2 : 1;
     // i-groups per CTA: at most an eighth of the i-block per CTA, so that a
     // mid-size block spreads over several i-tiles instead of one i-tile
-    // split many ways -- whose split fold (one thread per i over all splits)
-    // then dominates.  Measured at nj = 262144 (mixed): ni = 256 0.12 vs
-    // 0.31 ms, ni = 1024 0.39 vs 0.43 ms; ni >= 2048 unchanged (8 groups).
+    // split many ways, whose split fold then dominates.  Measured at nj =
+    // 262144 (mixed, with one thread per i over all splits; fold_splits has
+    // shortened the fold since): ni = 256 0.12 vs 0.31 ms, ni = 1024 0.39 vs
+    // 0.43 ms; ni >= 2048 unchanged (8 groups).
     int groups_needed = (ni + c.il * c.r - 1) / (c.il * c.r);
     int G = 1;
     while (G * 2 <= c.warps && G * 2 * 8 <= groups_needed) G *= 2;
